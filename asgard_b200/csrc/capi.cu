@@ -65,16 +65,10 @@ void free_plan(plan_data &p)
   cudaFree(p.gseg);
   cudaFree(p.gcell_order);
   cudaFree(p.gx32);
-  cudaFree(p.gjobs);
-  cudaFree(p.gchain_last);
-  cudaFree(p.gd_ptr);
-  cudaFree(p.gd_col);
-  cudaFree(p.gd_conn);
-  cudaFree(p.gd_rel);
-  cudaFree(p.gwork);
   cudaFree(p.vP64);
   cudaFree(p.vP32);
   tc_free(p.tc);
+  sweep_free(p.sweep);
   p = plan_data{};
 }
 
@@ -161,33 +155,6 @@ int global_blocks(int d, int terms, std::vector<int> const &conn_row,
         B[(j * d + k) * 10 + e] += blk(j, t, k)[e];
   }
   return ASGK_OK;
-}
-
-// The chains of a term acting in m >= 2 dimensions a_0 < ... < a_{m-1}, as
-// the reference's permutes (src/device/asgard_kronmult.hpp:152-224) builds
-// them: 2^(m-1) chains; in chain c, dimension a_s (s >= 1) takes the lower
-// part of its operator when bit s-1 of c is 0, the upper part (diagonal
-// included) when 1; a chain applies its upper parts first (in decreasing
-// order of s), then the whole operator of a_0, then its lower parts (in
-// increasing order of s).  The chains' sum is the term's operator on the
-// sparse grid.  Stage entries: (dimension, fill) with fill 0 = upper,
-// 1 = both, 2 = lower.
-std::vector<std::vector<std::pair<int, int>>> term_chains(std::vector<int> const &dims)
-{
-  int const m = int(dims.size());
-  std::vector<std::vector<std::pair<int, int>>> out;
-  for (int c = 0; c < (1 << (m - 1)); c++)
-  {
-    std::vector<int> signed_dir(m, 0); // -s: upper, +s: lower, 0: both
-    for (int s = 1; s < m; s++)
-      signed_dir[s] = ((c >> (s - 1)) & 1) ? -s : s;
-    std::sort(signed_dir.begin(), signed_dir.end());
-    std::vector<std::pair<int, int>> chain;
-    for (int v : signed_dir)
-      chain.emplace_back(dims[std::abs(v)], v < 0 ? 0 : (v > 0 ? 2 : 1));
-    out.push_back(chain);
-  }
-  return out;
 }
 
 int upload_global_blocks(plan_data &p, std::vector<double> const &B)
@@ -297,11 +264,123 @@ int alloc_plan(plan_data &p, int d, int n, int rows, int cols, int terms,
   return ASGK_OK;
 }
 
-// Builds the device plan from host CSR arrays (validated here).
+// The cells and the 1D connectivity behind a pair list: 1D indices per cell
+// (< R) and the connection of two 1D cells (row, column), -1 for none.
+struct grid_cells
+{
+  int R = 0;
+  std::vector<int> oned, lut;
+};
+
+// Whether a square pair list is that of a grid's whole connectivity: every
+// pair of its cells that is connected in all dimensions, once each, with the
+// factors of the 1D connections numbered as asgk_connect_1d numbers them (the
+// lists asgk_build_pairs and make_kronmult_sparse make,
+// src/asgard_kronmult_matrix.cpp:406-466).  conn(p, k): the connection of
+// pair p in dimension k, or -1.
+template<typename F>
+bool find_grid(int d, int rows, std::vector<int64_t> const &row_ptr, const int *col,
+               int64_t nconn, F &&conn, grid_cells &g)
+{
+  // the count of connected cells below compares every two cells
+  if (rows < 1 || rows > (1 << 15))
+    return false;
+  int nc = 0;
+  for (int level = 0; level <= 12 && nc < nconn; level++)
+    if (asgk_connect_1d(level, &g.R, &nc, nullptr, nullptr))
+      return false;
+  if (nc != nconn)
+    return false;
+  int level = 0;
+  while ((1 << level) < g.R)
+    ++level;
+  std::vector<int> pntr(g.R + 1), indx(nc), row_of(nc);
+  asgk_connect_1d(level, &g.R, &nc, pntr.data(), indx.data());
+  g.lut.assign(size_t(g.R) * g.R, -1);
+  for (int r = 0; r < g.R; r++)
+    for (int j = pntr[r]; j < pntr[r + 1]; j++)
+    {
+      row_of[j]                        = r;
+      g.lut[size_t(r) * g.R + indx[j]] = j;
+    }
+  g.oned.resize(size_t(rows) * d);
+  for (int r = 0; r < rows; r++)
+    for (int k = 0; k < d; k++)
+    {
+      int const j = row_ptr[r] < row_ptr[r + 1] ? conn(row_ptr[r], k) : -1;
+      if (j < 0)
+        return false;
+      g.oned[size_t(r) * d + k] = row_of[j];
+    }
+  bool ok = true;
+#pragma omp parallel
+  {
+    std::vector<int> seen(rows, -1);
+#pragma omp for schedule(dynamic, 16)
+    for (int r = 0; r < rows; r++)
+    {
+      bool good     = true;
+      const int *er = &g.oned[size_t(r) * d];
+      for (int64_t p = row_ptr[r]; p < row_ptr[r + 1] && good; p++)
+      {
+        const int *ec = &g.oned[size_t(col[p]) * d];
+        good          = seen[col[p]] != r;
+        seen[col[p]]  = r;
+        for (int k = 0; k < d && good; k++)
+          good = g.lut[size_t(er[k]) * g.R + ec[k]] >= 0 &&
+                 conn(p, k) == g.lut[size_t(er[k]) * g.R + ec[k]];
+      }
+      int64_t connected = 0;
+      for (int c = 0; c < rows && good; c++)
+      {
+        const int *ec = &g.oned[size_t(c) * d];
+        bool on       = true;
+        for (int k = 0; k < d && on; k++)
+          on = g.lut[size_t(er[k]) * g.R + ec[k]] >= 0;
+        connected += on ? 1 : 0;
+      }
+      if (!good || connected != row_ptr[r + 1] - row_ptr[r])
+#pragma omp atomic write
+        ok = false;
+    }
+  }
+  return ok;
+}
+
+// Gives an allocated pair plan the tree of 1D passes over its grid
+// (kron_sweep.cu), which then computes its applies.  A grid that the tree
+// does not reach all cells of, or too little memory for its vectors, leaves
+// the plan with the pair kernels.
+int attach_sweep(plan_data &p, grid_cells const &g)
+{
+  std::vector<std::vector<int>> terms(p.terms);
+  for (int t = 0; t < p.terms; t++)
+  {
+    terms[t].push_back(t);
+    for (int k = 0; k < p.d; k++)
+      terms[t].push_back(k);
+  }
+  int rc = ASGK_OK;
+  if (p.vP64 == nullptr) // the expanded form
+  {
+    int64_t const blk = int64_t(p.d) * p.terms * 9;
+    if ((rc = dev_alloc(&p.vP64, p.vA_len / blk * p.d * p.terms * 10, p.device_bytes)) == ASGK_OK)
+      rc = dev_alloc(&p.vP32, p.vA_len / blk * p.d * p.terms * 12, p.device_bytes);
+    if (rc == ASGK_OK)
+      p.nconn = p.vA_len / blk;
+  }
+  if (rc == ASGK_OK)
+    rc = sweep_build(p.d, p.rows, g.oned.data(), g.lut.data(), g.R, terms, true, &p.sweep,
+                     p.device_bytes);
+  return (rc == ASGK_ERR_UNSUPPORTED || rc == ASGK_ERR_ALLOC) ? int(ASGK_OK) : rc;
+}
+
+// Builds the device plan from host CSR arrays (validated here).  grid: the
+// cells behind the list when the caller knows that it is complete.
 int build_plan(asgk_plan **out, int d, int n, int rows, int cols, int terms,
                std::vector<int64_t> const &row_ptr, const int *col,
                const int *idx, index_mode mode, const double *vA,
-               int64_t vA_len)
+               int64_t vA_len, grid_cells const *grid = nullptr, bool diagonal = false)
 {
   if (out == nullptr)
     return ASGK_ERR_INVALID;
@@ -360,14 +439,39 @@ int build_plan(asgk_plan **out, int d, int n, int rows, int cols, int terms,
     ASGK_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
     return ASGK_OK;
   };
+  if (n == 3 && d >= 2 && rows == cols && !diagonal && sweep_pays(d, nnz * terms, false))
+  {
+    grid_cells found;
+    auto conn_of = [&](int64_t q, int k) { return idx[q * d + k]; };
+    auto offset_conn = [&](int64_t q, int k) {
+      // one 1D connection behind the offsets of all terms
+      int const *ia   = idx + q * terms * d + k;
+      int64_t const j = (int64_t(ia[0]) - int64_t(k) * 9) / blk;
+      for (int t = 0; t < terms; t++)
+        if (ia[int64_t(t) * d] != j * blk + int64_t(t * d + k) * 9)
+          return -1;
+      return int(j);
+    };
+    if (grid == nullptr && vA_len % blk == 0 &&
+        (mode == index_mode::conn ? find_grid(d, rows, row_ptr, col, vA_len / blk, conn_of, found)
+                                  : find_grid(d, rows, row_ptr, col, vA_len / blk, offset_conn, found)))
+      grid = &found;
+    if (grid != nullptr && (rc = attach_sweep(p, *grid)))
+    {
+      free_plan(p);
+      return rc;
+    }
+  }
   // For the staged n = 3, d = 3/4 kernel, each row's pairs are ordered by
   // their factor blocks, the last dimension slowest and dimension 0 fastest:
   // the ten pairs a warp contracts together then mostly share the blocks of
   // dimensions 1..d-1 (read whole) and differ in dimension 0 (read as one
   // column per lane), and a block's reuse distance stays within L1.  The
-  // result changes only by the order of the floating-point sums.
+  // result changes only by the order of the floating-point sums.  (A plan
+  // that the tree applies in both precisions needs no order.)
   std::vector<int> col_sorted, idx_sorted;
-  if (n == 3 && (d == 3 || d == 4) && terms > 0 && nnz > 0)
+  if (n == 3 && (d == 3 || d == 4) && terms > 0 && nnz > 0 && !diagonal &&
+      !(p.sweep != nullptr && sweep_pays(d, nnz * terms, true)))
   {
     int64_t const per = (mode == index_mode::conn) ? d : int64_t(terms) * d;
     col_sorted.resize(nnz);
@@ -1358,9 +1462,20 @@ int asgk_plan_create_dense(asgk_plan **plan, int d, int n, int num_rows,
     std::vector<double> vA;
     if (num_terms > 0)
       vA = dense_values(d, n, num_terms, nb, terms);
+    // rows and columns the same cells: a grid whose 1D cells are all connected
+    grid_cells g;
+    if (num_rows == num_cols && row_offset == col_offset && npairs > 0 && nb <= 4096)
+    {
+      g.R = nb;
+      g.oned.assign(elem + int64_t(row_offset) * d, elem + int64_t(row_offset + num_rows) * d);
+      g.lut.resize(size_t(nb) * nb);
+      for (int r = 0; r < nb; r++)
+        for (int c = 0; c < nb; c++)
+          g.lut[size_t(r) * nb + c] = c * nb + r;
+    }
     if (int rc = build_plan(plan, d, n, num_rows, num_cols, num_terms, rp,
                             col.data(), conn.data(), index_mode::conn,
-                            vA.data(), int64_t(vA.size())))
+                            vA.data(), int64_t(vA.size()), g.R > 0 ? &g : nullptr))
       return rc;
     (*plan)->p.dense    = true;
     (*plan)->p.dense_nb = nb;
@@ -1520,6 +1635,14 @@ int asgk_plan_create_grid(asgk_plan **plan, int d, int n, int level,
     if (!rc && nnz > 0)
       rc = launch_fill_pairs(d, cells, d_oned, d_cand, d_lut, R, p.row_ptr, p.col,
                              p.idx, nullptr);
+    if (!rc && n == 3 && d >= 2 && sweep_pays(d, nnz * num_terms, false))
+    {
+      grid_cells g;
+      g.R    = R;
+      g.oned = std::move(oned);
+      g.lut  = std::move(lut);
+      rc     = attach_sweep(p, g);
+    }
     if (!rc)
       rc = upload_values(p, vA);
     release();
@@ -1599,7 +1722,7 @@ int asgk_plan_update_values(asgk_plan *plan, const double *vA, int64_t vA_len)
       if (int rc = global_blocks(p.d, p.terms, p.g_conn_row, p.g_conn_col, vA, B,
                                  n_identity, multi))
         return rc;
-      // the chains are built for the dimensions each term acts in
+      // the sweeps are built for the dimensions each term acts in
       if (multi != p.g_multi)
         return ASGK_ERR_INVALID;
       if (int rc = upload_global_blocks(p, B))
@@ -1678,7 +1801,7 @@ int asgk_plan_create_global(asgk_plan **plan, int d, int n, int level,
         conn[size_t(r) * d + k] = dp.self_conn[size_t(r) * d + k];
     }
     if (int rc = build_plan(plan, d, n, num_cells, num_cells, num_terms, rp,
-                            col.data(), conn.data(), index_mode::conn, vA, vA_len))
+                            col.data(), conn.data(), index_mode::conn, vA, vA_len, nullptr, true))
       return rc;
     auto &p = (*plan)->p;
     p.global     = true;
@@ -1741,79 +1864,32 @@ int asgk_plan_create_global(asgk_plan **plan, int d, int n, int level,
       *plan = nullptr;
       return rc;
     }
-    // chains of the terms acting in several dimensions
+    // the terms acting in several dimensions
     p.g_multi = multi;
     if (!multi.empty())
     {
-      std::vector<std::vector<std::pair<int, int>>> chains;
-      std::vector<int> chain_term;
-      for (auto const &m : multi)
-        for (auto &c : term_chains(std::vector<int>(m.begin() + 1, m.end())))
-        {
-          chains.push_back(c);
-          chain_term.push_back(m[0]);
-        }
-      p.gchains = int(chains.size());
-      int stages = 0;
-      for (auto const &c : chains)
-        stages = std::max(stages, int(c.size()));
-      // per-dimension neighbour lists (every entry of the direction pairs)
-      std::vector<int64_t> dptr(size_t(d) * (num_cells + 1), 0);
-      std::vector<int> dcol, dconn;
-      std::vector<unsigned char> drel;
-      std::vector<int64_t> per_dim(d, 0);
-      for (int k = 0; k < d; k++)
-      {
-        for (int r = 0; r < num_cells; r++)
-        {
-          for (int64_t e = dp.ptr[r]; e < dp.ptr[r + 1]; e++)
-            if (dp.dim[e] == k)
-            {
-              int const j = dp.conn[e];
-              dcol.push_back(dp.col[e]);
-              dconn.push_back(j);
-              drel.push_back(dp.conn_col[j] < dp.conn_row[j] ? 0 : (dp.conn_col[j] == dp.conn_row[j] ? 1 : 2));
-            }
-          dptr[size_t(k) * (num_cells + 1) + r + 1] = int64_t(dcol.size());
-        }
-        per_dim[k] = int64_t(dcol.size()) - dptr[size_t(k) * (num_cells + 1)];
-        if (k + 1 < d)
-          dptr[size_t(k + 1) * (num_cells + 1)] = int64_t(dcol.size());
-      }
-      std::vector<int4> jobs;
-      for (int s = 0; s < stages; s++)
-      {
-        p.stage_job0.push_back(int(jobs.size()));
-        for (int c = 0; c < p.gchains; c++)
-          if (int(chains[c].size()) > s)
-          {
-            jobs.push_back(make_int4(c, chains[c][s].first, chains[c][s].second, chain_term[c]));
-            p.gchain_entries += per_dim[chains[c][s].first];
-          }
-        p.stage_njobs.push_back(int(jobs.size()) - p.stage_job0.back());
-      }
-      std::vector<int> last(p.gchains);
-      for (int c = 0; c < p.gchains; c++)
-        last[c] = (int(chains[c].size()) - 1) % 2;
-      int64_t const N = int64_t(num_cells) * p.tensor;
-      if ((rc = dev_alloc(&p.gjobs, int64_t(jobs.size()), bytes)) ||
-          (rc = dev_alloc(&p.gchain_last, p.gchains, bytes)) ||
-          (rc = dev_alloc(&p.gd_ptr, int64_t(dptr.size()), bytes)) ||
-          (rc = dev_alloc(&p.gd_col, std::max<int64_t>(int64_t(dcol.size()), 1), bytes)) ||
-          (rc = dev_alloc(&p.gd_conn, std::max<int64_t>(int64_t(dconn.size()), 1), bytes)) ||
-          (rc = dev_alloc(&p.gd_rel, std::max<int64_t>(int64_t(drel.size()), 1), bytes)) ||
-          (rc = dev_alloc(&p.gwork, 2 * int64_t(p.gchains) * N, bytes)) ||
-          (rc = up(p.gjobs, jobs.data(), sizeof(int4) * jobs.size())) ||
-          (rc = up(p.gchain_last, last.data(), sizeof(int) * last.size())) ||
-          (rc = up(p.gd_ptr, dptr.data(), sizeof(int64_t) * dptr.size())) ||
-          (rc = up(p.gd_col, dcol.data(), sizeof(int) * dcol.size())) ||
-          (rc = up(p.gd_conn, dconn.data(), sizeof(int) * dconn.size())) ||
-          (rc = up(p.gd_rel, drel.data(), drel.size())))
+      int R = 0;
+      for (int r : dp.conn_row)
+        R = std::max(R, r + 1);
+      std::vector<int> lut(size_t(R) * R, -1), oned(size_t(num_cells) * d);
+      for (int j = 0; j < dp.nconn; j++)
+        lut[size_t(dp.conn_row[j]) * R + dp.conn_col[j]] = j;
+      for (size_t i = 0; i < oned.size(); i++)
+        oned[i] = dp.conn_row[dp.self_conn[i]];
+      if ((rc = sweep_build(d, num_cells, oned.data(), lut.data(), R, multi, false, &p.sweep,
+                            bytes)))
       {
         asgk_plan_destroy(*plan);
         *plan = nullptr;
         return rc;
       }
+      // a term of m dimensions is 2^(m-1) upper/lower chains of m passes
+      std::vector<int64_t> per_dim(d, 0);
+      for (int k : dp.dim)
+        ++per_dim[k];
+      for (auto const &m : multi)
+        for (size_t i = 1; i < m.size(); i++)
+          p.gchain_entries += per_dim[m[i]] << (m.size() - 2);
     }
     // d >= 5: per-cell dimension segments (the entries of a cell come in
     // dimension order) and two cell orders
@@ -2314,7 +2390,7 @@ int gmres_euler_impl(asgk_plan *plan, double dt, double *x, const double *b,
   // kernel of a step reads the gate: the global operator without chains
   // (one kernel), a Jacobi preconditioner or none, the Krylov kernels
   int const node_steps =
-      (p.global && p.gchains == 0 && p.terms > 0 && p.nnz > 0 && dt != 0.0)
+      (p.global && p.g_multi.empty() && p.terms > 0 && p.nnz > 0 && dt != 0.0)
           ? g_gmres_node_steps
           : 1;
 

@@ -78,6 +78,8 @@ enum class index_mode : int
 
 // kron_tc.cu: the tensor-core (BF16) form of a global plan's operator
 struct tc_data;
+// kron_sweep.cu: the tree of 1D passes of terms acting in several dimensions
+struct sweep_data;
 
 // Device-resident operator.  Pairs are grouped by output cell (CSR) and the
 // cells are visited in order of decreasing pair count.
@@ -140,22 +142,15 @@ struct plan_data
   // the vector whose FP32 copy gx32 holds when a preconditioner wrote it
   // with its output (consumed, and cleared, by the next FP32 global apply)
   mutable const double *gx32_src = nullptr;
-  // terms acting in several dimensions (the reference's upper/lower
-  // permutations): chains of masked 1D passes over per-dimension neighbour
-  // lists.  Stage s runs the jobs gjobs[stage_job0[s] ..] (chain, dimension,
-  // fill 0 upper / 1 both / 2 lower, term); chain outputs alternate between
-  // two buffers of gchains vectors, chain c's result is in buffer
-  // gchain_last[c].
-  std::vector<std::vector<int>> g_multi; // (term, its dimensions) per such term
-  int gchains = 0;
-  std::vector<int> stage_job0, stage_njobs;
-  int4 *gjobs = nullptr;
-  int *gchain_last = nullptr;
-  int64_t *gd_ptr = nullptr;       // [d][rows + 1]
-  int *gd_col = nullptr, *gd_conn = nullptr;
-  unsigned char *gd_rel = nullptr; // neighbour's 1D cell: 0 before, 1 same, 2 after
-  double *gwork = nullptr;         // 2 * gchains * rows * n^d values
-  int64_t gchain_entries = 0;      // neighbour entries the chains' stages visit
+  // global mode: the terms acting in several dimensions, each as (term, its
+  // dimensions), and the neighbour entries that their separate upper/lower
+  // chains (the reference's permutes) visit, which asgk_plan_info reports
+  std::vector<std::vector<int>> g_multi;
+  int64_t gchain_entries = 0;
+  // the tree of 1D passes of terms acting in several dimensions: those of a
+  // global plan, or every term of a pair plan whose list holds all connected
+  // pairs of its cells (null: the pair kernels)
+  sweep_data *sweep = nullptr;
 
   // the tensor-core form of a global plan (precision ASGK_BF16): pencils,
   // their BF16 class matrices and its vectors, built on first use
@@ -243,6 +238,29 @@ int line_info(line_data const &ld, int *dims);
 int launch_global(plan_data const &p, int precision, double alpha,
                   const double *x, double beta, double *y, double ex,
                   cudaStream_t s);
+
+// kron_sweep.cu: terms acting in several dimensions as a tree of 1D passes.
+// Vectors the tree may hold at once (beyond what one path needs).
+constexpr int64_t kSweepBytes = int64_t(3) << 29;
+int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
+                std::vector<std::vector<int>> const &terms, bool require_closed,
+                sweep_data **out, int64_t &bytes);
+void sweep_free(sweep_data *w);
+// Whether a pair plan of `products` pairs x terms in d dimensions is applied
+// by the tree rather than by the pair kernels.  The tree costs 2d launches
+// of 4-10 us, the pair kernels one whose time grows with the products; both
+// measured with FP64 on either side of the line: d=2 level 7, 155 and 464
+// thousand products: tree 18 and 24 us, pairs 15 and 28; d=3, 188 and 1058:
+// 32 and 37, 22 and 64; d=4, 107 and 276: 43 and 47, 31 and 60; d=5, 55 and
+// 101: 66 and 62, 56 and 94; d=6, 57 and 247: 129 and 157, 119 and 475.  The
+// pair kernels gain more from FP32.
+inline bool sweep_pays(int d, int64_t products, bool fp32)
+{
+  int64_t const least = d <= 3 ? 400000 : (d == 4 ? 262144 : 65536);
+  return products >= (fp32 ? least * 3 / 2 : least);
+}
+int launch_sweep(plan_data const &p, sweep_data const &w, int precision, double alpha,
+                 const void *x, bool f32, double beta, void *y, double ex, cudaStream_t s);
 
 // kron_tc.cu: the tensor-core form (tcgen05, BF16 operands, FP32 TMEM
 // accumulators) of a global plan whose terms act in one dimension each.

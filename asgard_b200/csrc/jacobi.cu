@@ -719,7 +719,7 @@ int jacobi_build(plan_data const &p, double dt, int kind, jacobi_data &jd)
     return ASGK_ERR_UNSUPPORTED; // the shared-memory inverse holds ts x 2ts
   // the Kronecker-sum form needs the global form's per-dimension blocks and
   // no term acting in several dimensions
-  if (kind == ASGK_JACOBI_KRON && (!p.global || p.gchains > 0 || p.n != 3))
+  if (kind == ASGK_JACOBI_KRON && (!p.global || !p.g_multi.empty() || p.n != 3))
     return ASGK_ERR_UNSUPPORTED;
   static std::atomic<uint64_t> next_serial{1};
   jd.serial = next_serial.fetch_add(1);

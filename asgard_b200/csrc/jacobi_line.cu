@@ -1107,7 +1107,7 @@ void line_free(line_data *ld) { delete ld; }
 int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
 {
   *out = nullptr;
-  if (!p.global || p.gchains > 0 || p.n != 3 || p.rows != p.cols)
+  if (!p.global || !p.g_multi.empty() || p.n != 3 || p.rows != p.cols)
     return ASGK_ERR_UNSUPPORTED;
   int const d         = p.d;
   int64_t const nconn = int64_t(p.g_conn_row.size());

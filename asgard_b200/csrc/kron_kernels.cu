@@ -469,6 +469,10 @@ int launch_apply(plan_data const &p, int precision, double alpha,
                          beta, static_cast<double *>(y), ex, s);
   }
   bool const euler = (ex != 0.0);
+  // every connected pair of a grid's cells: the tree of 1D passes
+  if (p.sweep != nullptr && (x_is_f32 != 0) == (y_is_f32 != 0) &&
+      sweep_pays(p.d, p.nnz * p.terms, x_is_f32 || precision == ASGK_FP32))
+    return launch_sweep(p, *p.sweep, precision, alpha, x, x_is_f32 != 0, beta, y, ex, s);
   if (x_is_f32 && y_is_f32)
     return dispatch<float, float, float>(p, p.vA32, alpha,
                                          static_cast<const float *>(x), beta,

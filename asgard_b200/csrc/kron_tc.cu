@@ -606,7 +606,7 @@ int tc_read_error(int reset, int *code)
 int tc_build(plan_data const &p, tc_data **out)
 {
   *out = nullptr;
-  if (!p.global || p.gchains > 0 || p.n != 3 || p.rows != p.cols || p.d < 1 || p.d > 6)
+  if (!p.global || !p.g_multi.empty() || p.n != 3 || p.rows != p.cols || p.d < 1 || p.d > 6)
     return ASGK_ERR_UNSUPPORTED;
   int const d = p.d;
   int r1      = 0;
