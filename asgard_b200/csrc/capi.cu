@@ -8,6 +8,7 @@
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <numeric>
 
@@ -512,6 +513,41 @@ int build_plan(asgk_plan **out, int d, int n, int rows, int cols, int terms,
 }
 
 cudaStream_t as_stream(asgk_stream s) { return static_cast<cudaStream_t>(s); }
+
+// The memory pool behind the scratch of single calls, one per device.  The
+// device's own pool gives its memory back to the system at every
+// synchronisation and fetches it again at the next call (0.45 ms of a 1.35 ms
+// Gram-Schmidt step); this one keeps up to kPoolBytes.  Allocations and frees
+// are ordered on the callers' streams, so calls of several threads and
+// streams share it safely.  Null when the device has no pools.
+constexpr uint64_t kPoolBytes = uint64_t(64) << 20;
+cudaMemPool_t scratch_pool()
+{
+  constexpr int kDevices = 64;
+  static std::mutex mu;
+  static cudaMemPool_t pools[kDevices] = {};
+  static bool tried[kDevices]          = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices)
+    return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!tried[dev])
+  {
+    tried[dev] = true;
+    cudaMemPoolProps props{};
+    props.allocType     = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id   = dev;
+    cudaMemPool_t pool  = nullptr;
+    uint64_t keep       = kPoolBytes;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      pools[dev] = pool;
+    else
+      cudaGetLastError();
+  }
+  return pools[dev];
+}
 
 // y = beta*y + alpha*A*x for a dense column-major n x n matrix (one warp per row)
 __global__ void k_dense_gemv(int n, const double *__restrict__ A, double alpha,
@@ -2277,8 +2313,11 @@ int asgk_cgs_step(const double *V, int64_t ldv, int k, double *w, int64_t n,
     int const blocks = max_reduction_blocks();
     double *part     = nullptr;
     size_t const cnt = size_t(blocks) * (k + 1) + 1;
-    ASGK_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&part),
-                              sizeof(double) * cnt, s));
+    if (cudaMemPool_t pool = scratch_pool())
+      ASGK_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&part), sizeof(double) * cnt,
+                                        pool, s));
+    else
+      ASGK_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&part), sizeof(double) * cnt, s));
     double *nrm2 = part + size_t(blocks) * (k + 1);
     int used     = 0;
     int rc       = launch_multidot(V, ldv, k, w, n, part, &used, s);

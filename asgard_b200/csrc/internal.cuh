@@ -241,7 +241,7 @@ int launch_global(plan_data const &p, int precision, double alpha,
 
 // kron_sweep.cu: terms acting in several dimensions as a tree of 1D passes.
 // Vectors the tree may hold at once (beyond what one path needs).
-constexpr int64_t kSweepBytes = int64_t(3) << 29;
+constexpr int64_t kSweepBytes = int64_t(768) << 20;
 int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
                 std::vector<std::vector<int>> const &terms, bool require_closed,
                 sweep_data **out, int64_t &bytes);

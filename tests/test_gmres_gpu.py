@@ -301,3 +301,28 @@ def test_line_preconditioner_fused_fp32_copy(cuda, graphs):
     assert i_f.true_relres == i_s.true_relres
     # one conversion launch fewer per preconditioned operator apply
     assert lf < ls
+
+
+@pytest.mark.parametrize("n,ldv,off,k", [(1, 1, 0, 1), (2, 2, 0, 3), (511, 511, 0, 8), (512, 514, 0, 9),
+                                         (4097, 4097, 1, 16), (300000, 300001, 0, 7),
+                                         (300000, 300000, 1, 26), (303105, 303106, 0, 50)])
+def test_cgs_step_layouts(cuda, n, ldv, off, k):
+    """One Gram-Schmidt step over bases whose size, leading dimension or
+    address does not allow 16-byte loads, and over those that do: h, w and the
+    norm against NumPy.  h_j sums n products: |h_j - exact| <= n u |V_j| |w|
+    in the worst order, u = 2^-53; the bars below are that for blocked sums."""
+    import asgard_b200 as ab
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    buf = torch.rand(k * ldv + 1, dtype=torch.float64, device="cuda", generator=g) * 2 - 1
+    V = buf[off:off + k * ldv].view(k, ldv)
+    w = torch.rand(n + 1, dtype=torch.float64, device="cuda", generator=g)[off:off + n]
+    Vn, wn = V[:, :n].cpu().numpy(), w.cpu().numpy()
+    h_ref = Vn @ wn
+    h, nrm = ab.cgs_step(V, k, w)
+    scale = np.linalg.norm(Vn, axis=1) * np.linalg.norm(wn)
+    assert (np.abs(h.cpu().numpy() - h_ref) <= 1e-14 * scale + 1e-300).all()
+    w_ref = wn - Vn.T @ h.cpu().numpy()
+    size = np.abs(wn) + np.abs(Vn).T @ np.abs(h.cpu().numpy())
+    assert (np.abs(w.cpu().numpy() - w_ref) <= k * 2.3e-16 * size).all()
+    assert abs(nrm - np.linalg.norm(w.cpu().numpy())) <= 1e-13 * nrm
