@@ -2425,13 +2425,10 @@ int gmres_euler_impl(asgk_plan *plan, double dt, double *x, const double *b,
     return rc;
   double const tol_abs = (tol_mode == ASGK_TOL_REL) ? tol * bnorm : tol;
 
-  // recorded cycles take several Arnoldi steps per graph node when every
-  // kernel of a step reads the gate: the global operator without chains
-  // (one kernel), a Jacobi preconditioner or none, the Krylov kernels
-  int const node_steps =
-      (p.global && p.g_multi.empty() && p.terms > 0 && p.nnz > 0 && dt != 0.0)
-          ? g_gmres_node_steps
-          : 1;
+  // recorded cycles take several Arnoldi steps per graph node: every kernel
+  // of a step reads the gate (the operator's, a Jacobi preconditioner's, the
+  // Krylov kernels) unless the operator is a scaling only
+  int const node_steps = (p.terms > 0 && p.nnz > 0 && dt != 0.0) ? g_gmres_node_steps : 1;
 
   core_stats st;
   int status = ASGK_OK;

@@ -606,8 +606,8 @@ int launch_global(plan_data const &p, int precision, double alpha,
                   const double *x, double beta, double *y, double ex,
                   cudaStream_t s)
 {
-  if (p.n != 3 || (g_gate != nullptr && p.sweep != nullptr))
-    return ASGK_ERR_UNSUPPORTED; // the sweeps take no gate
+  if (p.n != 3)
+    return ASGK_ERR_UNSUPPORTED;
   // terms that are the identity in every dimension add n_identity * x
   double const ex_eff = ex + alpha * p.g_identity;
   int rc = ASGK_ERR_UNSUPPORTED;

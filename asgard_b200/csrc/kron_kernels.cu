@@ -158,8 +158,10 @@ __global__ void __launch_bounds__(NW * 32)
                const int *__restrict__ row_order, const int *__restrict__ col,
                const int *__restrict__ idx, const TC *__restrict__ vA,
                double alpha, const TX *__restrict__ x, double beta,
-               TY *__restrict__ y, double ex)
+               TY *__restrict__ y, double ex, const double *__restrict__ gate)
 {
+  if (gate_closed(gate))
+    return;
   // conn mode: vA is the repacked [conn][d][T][pad] array
   using S = shape3<D, HL>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -295,8 +297,10 @@ __global__ void __launch_bounds__(256)
                       const int *__restrict__ col, const int *__restrict__ idx,
                       const TC *__restrict__ vA, double alpha,
                       const TX *__restrict__ x, double beta,
-                      TY *__restrict__ y, double ex)
+                      TY *__restrict__ y, double ex, const double *__restrict__ gate)
 {
+  if (gate_closed(gate))
+    return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TC *X   = reinterpret_cast<TC *>(smem_raw);
   TC *B0  = X + ts;
@@ -369,17 +373,15 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-constexpr int kWarps = 4;
-
 template<int D, typename TC, typename TX, typename TY, index_mode MODE,
-         bool EULER>
-int launch3(plan_data const &p, const TC *vA, double alpha, const TX *x,
+         bool EULER, int NW>
+int launch3_warps(plan_data const &p, const TC *vA, double alpha, const TX *x,
             double beta, TY *y, double ex, cudaStream_t s)
 {
   constexpr int HL = lanes3<D>::value;
   using S          = shape3<D, HL>;
-  size_t const shm = size_t(kWarps) * S::G * S::BUF * sizeof(TC);
-  auto kern        = kron3_rows<D, HL, TC, TX, TY, MODE, EULER, kWarps>;
+  size_t const shm = size_t(NW) * S::G * S::BUF * sizeof(TC);
+  auto kern        = kron3_rows<D, HL, TC, TX, TY, MODE, EULER, NW>;
   if constexpr (MODE == index_mode::conn)
   {
     if constexpr (std::is_same_v<TC, double>)
@@ -394,11 +396,29 @@ int launch3(plan_data const &p, const TC *vA, double alpha, const TX *x,
         kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
     configured = true;
   }
-  kern<<<p.rows, kWarps * 32, shm, s>>>(p.terms, p.row_ptr, p.row_order,
-                                       p.col, p.idx, vA, alpha, x, beta, y,
-                                       ex);
+  kern<<<p.rows, NW * 32, shm, s>>>(p.terms, p.row_ptr, p.row_order, p.col, p.idx, vA, alpha, x,
+                                    beta, y, ex, g_gate);
   ASGK_LAUNCHED();
   return ASGK_OK;
+}
+
+// Warps per output cell: a cell's warps take its pairs in turn, one latency
+// per turn, so few cells (a block each and SMs to spare) take more warps.
+// Measured, 4 / 8 / 16 warps, FP64 unless stated: d=2 level 7 (576 cells, 3
+// terms) 27.7 / 23.2 / 21.1 us; d=3 level 5 (272 cells, FP32) 16.9 / 13.0 /
+// 12.7, level 6 (688 cells) 39.5 / 41.9 / 44.1; d=4 level 4 (192 cells, FP32)
+// 21.5 / 25.2 / 25.1; d=5 level 3 (96 cells) 33.3 / 27.2 / 44.2; d=6 level 3
+// (138 cells) 119 / 95 / 152, level 4 (501 cells) 1193 / 1219 / 1966.
+template<int D, typename TC, typename TX, typename TY, index_mode MODE,
+         bool EULER>
+int launch3(plan_data const &p, const TC *vA, double alpha, const TX *x,
+            double beta, TY *y, double ex, cudaStream_t s)
+{
+  if constexpr (D == 2)
+    return launch3_warps<D, TC, TX, TY, MODE, EULER, 16>(p, vA, alpha, x, beta, y, ex, s);
+  else if (p.rows <= (D == 3 ? 2 : 1) * 148)
+    return launch3_warps<D, TC, TX, TY, MODE, EULER, 8>(p, vA, alpha, x, beta, y, ex, s);
+  return launch3_warps<D, TC, TX, TY, MODE, EULER, 4>(p, vA, alpha, x, beta, y, ex, s);
 }
 
 template<typename TC, typename TX, typename TY, bool EULER>
@@ -417,7 +437,7 @@ int launch_generic(plan_data const &p, const TC *vA, double alpha, const TX *x,
     threads *= 2;
   kern<<<p.rows, threads, shm, s>>>(p.d, p.n, p.tensor, p.terms, int(p.mode),
                                     p.row_ptr, p.row_order, p.col, p.idx, vA,
-                                    alpha, x, beta, y, ex);
+                                    alpha, x, beta, y, ex, g_gate);
   ASGK_LAUNCHED();
   return ASGK_OK;
 }

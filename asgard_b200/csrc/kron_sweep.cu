@@ -334,8 +334,11 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
     k_sweep(const int4 *__restrict__ units, unit_tables tab,
             const int *__restrict__ index, const int4 *__restrict__ recs,
             const int4 *__restrict__ jobs, const TC *__restrict__ P, int T,
-            const TX *__restrict__ x, TC *__restrict__ work, int64_t N)
+            const TX *__restrict__ x, TC *__restrict__ work, int64_t N,
+            const double *__restrict__ gate)
 {
+  if (gate_closed(gate))
+    return;
   constexpr int TS = ipow3w(D), F = TS / 3;
   __shared__ TC part[kWarps][3][32];
   __shared__ __align__(16) TC stage[kSmall * kSmall * padW<TC>::value];
@@ -405,9 +408,11 @@ template<typename TC, typename TX, typename TY>
 __global__ void k_sweep_sum(int terms, const int *__restrict__ last,
                             const TC *__restrict__ work, int64_t N, double alpha,
                             const TX *__restrict__ x, double ex, double beta,
-                            TY *__restrict__ y)
+                            TY *__restrict__ y, const double *__restrict__ gate)
 {
   wait_previous();
+  if (gate_closed(gate))
+    return;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < N;
        i += int64_t(gridDim.x) * blockDim.x)
   {
@@ -446,13 +451,13 @@ int launch_d(sweep_data const &w, const TC *P, int T, double alpha, const TX *x,
     ASGK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<D, TC, TX>, static_cast<const int4 *>(w.units), tab,
                                  static_cast<const int *>(w.index),
                                  static_cast<const int4 *>(w.recs),
-                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N));
+                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N, g_gate));
     count_launch();
   }
   cfg.gridDim = dim3(int(std::min<int64_t>((w.N + 255) / 256, 148 * 8)));
   ASGK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep_sum<TC, TX, TY>, w.nresults,
                                static_cast<const int *>(w.last), static_cast<const TC *>(work),
-                               w.N, alpha, x, ex, beta, y));
+                               w.N, alpha, x, ex, beta, y, g_gate));
   count_launch();
   return ASGK_OK;
 }

@@ -326,3 +326,41 @@ def test_cgs_step_layouts(cuda, n, ldv, off, k):
     size = np.abs(wn) + np.abs(Vn).T @ np.abs(h.cpu().numpy())
     assert (np.abs(w.cpu().numpy() - w_ref) <= k * 2.3e-16 * size).all()
     assert abs(nrm - np.linalg.norm(w.cpu().numpy())) <= 1e-13 * nrm
+
+
+@pytest.mark.parametrize("plan", ["pairs d2", "pairs d3", "pairs d6", "whole grid", "several dimensions",
+                                  "n = 4"])
+def test_steps_per_node_on_every_operator_form(cuda, plan):
+    """Every operator kernel returns at once when its cycle has stopped: a
+    solve with 16 Arnoldi steps per graph node gives the iterates of one step
+    per node and of host-driven cycles, bit for bit."""
+    import asgard_b200 as ab
+    import torch
+    shape = {"pairs d2": (2, 6, 2, "advdiff", "pairs"), "pairs d3": (3, 4, 3, "advdiff", "pairs"),
+             "pairs d6": (6, 2, 6, "advdiff", "pairs"), "whole grid": (4, 5, 4, "advdiff", "pairs"),
+             "several dimensions": (3, 4, 2, "random", "global")}
+    if plan == "n = 4":
+        data = oracle.make_kronmult_data(2, 4, 20, 2, 9)
+        mat = ab.kronmult_matrix.from_csr(2, 4, 20, 20, 2, data["pntr"], data["indx"], data["iA"],
+                                          data["vA"])
+        dt = 1e-4
+    else:
+        d, L, T, kind, mode = shape[plan]
+        mat = ab.SparseGridOperator(d, L, T, kind=kind, seed=1).kronmult_matrix(mode=mode)
+        dt = 1e-5 if kind == "random" else 1e-3
+    g = torch.Generator(device="cuda").manual_seed(3)
+    b = torch.rand(mat.output_size(), dtype=torch.float64, device="cuda", generator=g) * 2 - 1
+    for precision in ("fp64", "fp32"):
+        got = []
+        for graphs, steps in ((True, 16), (True, 1), (False, 1)):
+            old = ab.gmres_settings(graphs=graphs, node_steps=steps)
+            try:
+                x = torch.zeros_like(b)
+                info = ab.simple_gmres_euler(dt, mat, x, b, 20, 100, 1e-11, tol_mode="rel",
+                                             precision=precision)
+            finally:
+                ab.gmres_settings(**old)
+            assert info.status == 0 and info.true_relres <= 1e-11
+            got.append((info.iterations, x))
+        assert len({it for it, _ in got}) == 1 and got[0][0] > 3
+        assert all(torch.equal(got[0][1], x) for _, x in got[1:])
