@@ -28,6 +28,7 @@
 // first factor also normalises v and writes its FP32 copy inside recorded
 // GMRES cycles; intermediates live in two vectors held by the
 // preconditioner; no atomics (each value belongs to exactly one unit).
+#include "cluster.cuh"
 #include "internal.cuh"
 
 #include <algorithm>
@@ -365,11 +366,129 @@ __device__ void dense_rows(const R *__restrict__ Mt, int Rr, int Rp, int G,
   }
 }
 
+// ---- large pencils over a cluster of CTAs
+//
+// A CTA that takes a 128-cell pencil alone streams its 384 x 384 matrix twice
+// (1.2 MB in FP32) at what one SM can read, 41 us at d=4 level 7 with nine
+// such CTAs.  A cluster of kSplit CTAs shares the pencil instead: each holds
+// all of the unit's values, reads only the matrix columns of its own rows,
+// and writes the rows of the first product to every CTA's shared memory.
+constexpr int kSplit      = 4;
+constexpr int kSplitItems = 32; // (4-row block, group) items of a CTA, a lane each
+constexpr int kSplitTile  = 64; // matrix rows per staged tile
+// The pencils that clusters take, multiples of 4 kSplit cells: all that the
+// small-pencil kernel leaves while the clusters are resident at once (no
+// third launch), else the long ones, else none.  Level 7 solves without
+// with clusters: d=2 1.55 and 1.15 ms, d=3 1.67 and 1.27, d=4 6.16 and 3.76;
+// d=5 level 6 4.23 and 3.73.  On large vectors the rest of a factor covers
+// the chain and the copies only cost: d=6 level 6 7.3 and 7.9 ms, level 7
+// 21.1 and 21.8.
+constexpr int kSplitMinM       = 64;
+constexpr int kSplitUnits      = 2 * 148 / kSplit;
+constexpr int64_t kSplitValues = 1 << 20;
+inline bool line_splits(int m)
+{
+  return m % (4 * kSplit) == 0 && 3 * m / (4 * kSplit) <= kSplitItems;
+}
+
+// dense_rows for the CTA's own rows r0 .. r0 + nr - 1 (multiples of 4): out
+// is every CTA's with ALL.  Lane: a (4-row block, group) item; warp: an
+// eighth of every tile's matrix rows, the eight sums added in order.  buf:
+// two tiles of kSplitTile x nr values, then the warps' sums.
+template<typename R, int NC, int NCP, bool ALL>
+__device__ void dense_rows_split(const R *__restrict__ Mt, int Rr, int Rp, int r0, int nr, int G,
+                                 const R *in, R *out, const R *__restrict__ theta, const R *lamc,
+                                 R shift, R dt, R *buf)
+{
+  constexpr int W  = kLineThreads / 32;
+  constexpr int TW = kSplitTile / W; // a warp's rows of a tile
+  int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int const nb    = nr / 4;
+  int const tiles = (Rr + kSplitTile - 1) / kSplitTile;
+  int const chunks = nr * int(sizeof(R)) / 16;
+  auto issue = [&](int tile) {
+    int const t0 = tile * kSplitTile;
+    int const nt = min(kSplitTile, Rr - t0);
+    R *dst       = buf + (tile & 1) * kSplitTile * nr;
+    for (int c = threadIdx.x; c < nt * chunks; c += kLineThreads)
+    {
+      int const t = c / chunks, q = c - t * chunks;
+      cp_async16(reinterpret_cast<char *>(dst + t * nr) + 16 * q,
+                 reinterpret_cast<const char *>(Mt + int64_t(t0 + t) * Rp + r0) + 16 * q);
+    }
+    cp_async_commit();
+  };
+  bool const has = lane < nb * G;
+  int const rb = has ? lane % nb : 0, g = has ? lane / nb : 0;
+  R acc[4][NC];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+      acc[i][c] = R(0);
+  issue(0);
+  for (int tile = 0; tile < tiles; tile++)
+  {
+    if (tile + 1 < tiles)
+    {
+      issue(tile + 1);
+      cp_async_wait<1>();
+    }
+    else
+      cp_async_wait<0>();
+    __syncthreads();
+    int const t0 = tile * kSplitTile + warp * TW;
+    const R *qt  = buf + (tile & 1) * kSplitTile * nr + warp * TW * nr + 4 * rb;
+#pragma unroll
+    for (int tt = 0; tt < TW; tt++)
+    {
+      if (t0 + tt >= Rr)
+        break;
+      R q[4], xv[NCP];
+      smem_row4(qt + tt * nr, q);
+      smem_row<R, NCP>(in + (int64_t(t0 + tt) * G + g) * NCP, xv);
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+      {
+        fma_pair(q[0], q[1], xv[c], acc[0][c], acc[1][c]);
+        fma_pair(q[2], q[3], xv[c], acc[2][c], acc[3][c]);
+      }
+    }
+    __syncthreads(); // the buffer is refilled two tiles on
+  }
+  int const values = nr * G * NC;
+  if (has)
+  {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int c = 0; c < NC; c++)
+        buf[warp * values + ((4 * rb + i) * G + g) * NC + c] = acc[i][c];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < values; e += kLineThreads)
+  {
+    int const rg = e / NC, c = e - rg * NC;
+    R v = buf[e];
+#pragma unroll
+    for (int w = 1; w < W; w++)
+      v += buf[w * values + e];
+    if (theta)
+      v = v / (shift - dt * (__ldg(theta + r0 + rg / G) + lamc[c]));
+    R *o = out + (int64_t(r0) * G + rg) * NCP + c;
+    if constexpr (ALL)
+      put_all<kSplit>(o, v);
+    else
+      *o = v;
+  }
+}
+
 // One factor M_k^-1 (after B when bj) on the (pencil, group range) units.
 // D dimensions, M line dimensions; NC = 3^(M-1) columns per group (the other
 // line dimensions' polynomials), groups: the 3^(D-M) polynomial indices of
-// the non-line dimensions.
-template<typename R, int D, int M, int KIDX>
+// the non-line dimensions.  CS > 1: a cluster of CS CTAs takes a unit, each
+// gathering, transforming and scattering the values of its own cells.
+template<typename R, int D, int M, int KIDX, int CS>
 __global__ void __launch_bounds__(kLineThreads)
     k_line_factor(line_args<R> a, const double *in64,
                   const R *__restrict__ inR, double *__restrict__ out64,
@@ -384,7 +503,7 @@ __global__ void __launch_bounds__(kLineThreads)
   constexpr int NCP = NC == 1 ? 1 : (NC == 3 ? 4 : 12);
   constexpr int NNL = D - M; // non-line dimensions
   extern __shared__ __align__(16) unsigned char line_smem[];
-  int4 const u   = a.units[blockIdx.x];
+  int4 const u   = a.units[blockIdx.x / CS];
   int const pen  = u.x, g0 = u.y, G = u.z;
   int const m    = a.pen_m[pen];
   int const tab  = a.pen_tab[pen];
@@ -398,7 +517,10 @@ __global__ void __launch_bounds__(kLineThreads)
   int *s_xrow       = reinterpret_cast<int *>(s_rowoff + m * G);
   R *X = reinterpret_cast<R *>(line_smem + ((12 * size_t(m) * G + 15) / 16) * 16);
   R *Y    = X + int64_t(Rp) * G * NCP;
-  R *qbuf = Y + int64_t(Rp) * G * NCP; // 2 tiles of kLineTile matrix rows
+  R *qbuf = Y + int64_t(Rp) * G * NCP; // matrix tiles (and the warps' sums)
+  // the CTA's own cells of the pencil
+  int const rank = CS > 1 ? cluster_rank() : 0;
+  int const i_lo = m / CS * rank, i_hi = CS > 1 ? i_lo + m / CS : m;
   __shared__ int s_offg[27];
   __shared__ int s_offc[NC];
   __shared__ R s_lamc[NC];
@@ -449,19 +571,28 @@ __global__ void __launch_bounds__(kLineThreads)
     s_rowoff[it] = int64_t(__ldg(cells + i)) * TS + s_offg[g];
     s_xrow[it]   = (i * 3 * G + g) * NCP;
   }
-  __syncthreads();
+  if constexpr (CS > 1)
+    cluster_sync(); // every CTA runs before its memory is written
+  else
+    __syncthreads();
   int const stk = ipow3l(D - 1 - a.k);
   double const f = scale_state ? scale_state[1] : 1.0;
   // gather (row = member * 3 + k polynomial, group, column); kGatherLoads
   // independent loads per thread are issued before their values are used
-  int const nload = m * G * 3 * NC;
+  int const e_lo = i_lo * G * 3 * NC, nload = i_hi * G * 3 * NC;
+  auto keep      = [&](int at, R val) {
+    if constexpr (CS > 1)
+      put_all<kSplit>(X + at, val);
+    else
+      X[at] = val;
+  };
   auto gidx = [&](int e, int &xo) {
     int const ig = e / (3 * NC), w = e - ig * (3 * NC);
     int const pk = w / NC, c = w - pk * NC;
     xo           = s_xrow[ig] + pk * G * NCP + c;
     return s_rowoff[ig] + s_offc[c] + pk * stk;
   };
-  for (int e0 = threadIdx.x; e0 < nload; e0 += kGatherLoads * kLineThreads)
+  for (int e0 = e_lo + threadIdx.x; e0 < nload; e0 += kGatherLoads * kLineThreads)
   {
     int64_t gi[kGatherLoads];
     int xo[kGatherLoads];
@@ -491,7 +622,7 @@ __global__ void __launch_bounds__(kLineThreads)
           if (vcopy)
             vcopy[gi[u]] = float(vv);
         }
-        X[xo[u]] = R(vv);
+        keep(xo[u], R(vv));
       }
     }
     else
@@ -504,10 +635,13 @@ __global__ void __launch_bounds__(kLineThreads)
 #pragma unroll
       for (int u = 0; u < kGatherLoads; u++)
         if (e0 + u * kLineThreads < nload)
-          X[xo[u]] = v[u];
+          keep(xo[u], v[u]);
     }
   }
-  __syncthreads();
+  if constexpr (CS > 1)
+    cluster_sync();
+  else
+    __syncthreads();
   // B = s - dt sum_{line j} S_j along j, on each (member, group): its 3 x NC
   // values are the cell's line-dimension polynomials
   if (bj)
@@ -563,10 +697,10 @@ __global__ void __launch_bounds__(kLineThreads)
     __syncthreads();
   }
   // columns: u <- P_j^T u along every other line dimension, per (row, group)
-  auto columns = [&](R *buf, bool forward) {
+  auto columns = [&](R *buf, bool forward, int rlo, int rhi) {
     if constexpr (NC > 1)
     {
-      for (int it = threadIdx.x; it < Rr * G; it += blockDim.x)
+      for (int it = rlo * G + threadIdx.x; it < rhi * G; it += blockDim.x)
       {
         R *row = buf + int64_t(it) * NCP;
         R v[NC];
@@ -604,18 +738,30 @@ __global__ void __launch_bounds__(kLineThreads)
       __syncthreads();
     }
   };
-  columns(X, true);
+  columns(X, true, 0, Rr);
   int64_t const to = a.tab_off[tab];
   // rows: Y = Q^T X, divided; then X = Q Y
-  dense_rows<R, NC, NCP>(a.Q + to, Rr, Rp, G, X, Y, a.theta + a.tab_th[tab], s_lamc,
-                         a.shift, a.dt, qbuf);
+  if constexpr (CS > 1)
+  {
+    int const r0 = 3 * i_lo, nr = 3 * (i_hi - i_lo);
+    dense_rows_split<R, NC, NCP, true>(a.Q + to, Rr, Rp, r0, nr, G, X, Y, a.theta + a.tab_th[tab],
+                                       s_lamc, a.shift, a.dt, qbuf);
+    cluster_sync();
+    dense_rows_split<R, NC, NCP, false>(a.QT + to, Rr, Rp, r0, nr, G, Y, X, nullptr, s_lamc,
+                                        a.shift, a.dt, qbuf);
+  }
+  else
+  {
+    dense_rows<R, NC, NCP>(a.Q + to, Rr, Rp, G, X, Y, a.theta + a.tab_th[tab], s_lamc,
+                           a.shift, a.dt, qbuf);
+    __syncthreads();
+    dense_rows<R, NC, NCP>(a.QT + to, Rr, Rp, G, Y, X, nullptr, s_lamc, a.shift,
+                           a.dt, qbuf);
+  }
   __syncthreads();
-  dense_rows<R, NC, NCP>(a.QT + to, Rr, Rp, G, Y, X, nullptr, s_lamc, a.shift,
-                         a.dt, qbuf);
-  __syncthreads();
-  columns(X, false);
+  columns(X, false, 3 * i_lo, 3 * i_hi);
   // scatter
-  for (int e = threadIdx.x; e < nload; e += blockDim.x)
+  for (int e = e_lo + threadIdx.x; e < nload; e += blockDim.x)
   {
     int xo;
     int64_t const gi = gidx(e, xo);
@@ -1037,6 +1183,9 @@ struct line_factor
 {
   int k = 0;
   int nunits = 0;   // (pencil, group range) units of the larger pencils
+  int nsplit = 0;   // the first of them, a cluster each
+  int split_rows = 0, split_tile = 0; // their largest Rp * G; rows per CTA
+  int split_sums = 0;                 // and rows per CTA * groups
   int max_rows = 0; // largest Rp * G of its units (shared memory)
   int max_rp   = 0; // largest padded pencil size (matrix tiles)
   int nbatches = 0; // batches of pencils of 1, 2, 4 or 8 cells
@@ -1078,11 +1227,12 @@ struct line_data
   line_tables<float> t32;
   std::vector<std::unique_ptr<line_factor>> factors;
   double *work = nullptr; // two intermediate vectors (rows * ts doubles each)
-  // a factor's small-pencil and larger-pencil launches touch disjoint cells:
-  // the larger ones run on a second stream, forked from and joined back to
-  // the caller's (parallel branches when the caller records a graph)
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork[3] = {nullptr, nullptr, nullptr}, join[3] = {nullptr, nullptr, nullptr};
+  // a factor's small-pencil, larger-pencil and cluster launches touch disjoint
+  // cells: the latter two run on streams of their own, forked from and joined
+  // back to the caller's (parallel branches when the caller records a graph)
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t fork[3] = {nullptr, nullptr, nullptr}, join[3] = {nullptr, nullptr, nullptr},
+              join2[3] = {nullptr, nullptr, nullptr};
   ~line_data()
   {
     for (int q = 0; q < 3; q++)
@@ -1091,9 +1241,13 @@ struct line_data
         cudaEventDestroy(fork[q]);
       if (join[q])
         cudaEventDestroy(join[q]);
+      if (join2[q])
+        cudaEventDestroy(join2[q]);
     }
     if (side)
       cudaStreamDestroy(side);
+    if (side2)
+      cudaStreamDestroy(side2);
     cudaFree(c1);
     cudaFree(tab_off);
     cudaFree(tab_th);
@@ -1295,9 +1449,24 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
       pen_tab.swap(o_tab);
     }
     auto small = [](int m) { return m == 1 || m == 2 || m == 4 || m == kSmallMaxM; };
+    int split_min = 0; // the pencils of at least this many cells go to clusters
+    for (int least : {2 * kSmallMaxM, kSplitMinM})
+    {
+      int64_t clusters = 0;
+      for (int m : pen_m)
+        if (m >= least && line_splits(m))
+        {
+          int const G = kSplitItems / (3 * m / (4 * kSplit));
+          clusters += (ng + G - 1) / G;
+        }
+      if (split_min == 0 && clusters <= kSplitUnits &&
+          int64_t(p.rows) * p.tensor <= kSplitValues)
+        split_min = least;
+    }
+    auto split = [&](int m) { return split_min > 0 && m >= split_min && line_splits(m); };
     int rpmax = 0;
     for (size_t pe = 0; pe < pen_m.size(); pe++)
-      if (!small(pen_m[pe]))
+      if (!small(pen_m[pe]) && !split(pen_m[pe]))
         rpmax = std::max(rpmax, trp[pen_tab[pe]]);
     // a unit's (4-row block, group) items: at most two per item slot; its
     // rows x groups bound its shared memory
@@ -1305,6 +1474,7 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
     int max_rp       = 0;
     std::vector<int4> units, batches, bcells;
     int max_rows = 0;
+    int nsplit = 0, split_rows = 0, split_tile = 0, split_sums = 0;
     for (size_t pe = 0; pe < pen_m.size();)
     {
       int const m = pen_m[pe];
@@ -1332,6 +1502,22 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
         continue;
       }
       int const Rp = trp[pen_tab[pe]];
+      int const nb = 3 * m / (4 * kSplit); // 4-row blocks of a cluster's CTA
+      if (split(m))
+      {
+        // (the pencils come in decreasing size: these units are the first)
+        int const G = std::min(std::min(ng, 27), kSplitItems / nb);
+        for (int g0 = 0; g0 < ng; g0 += G)
+        {
+          int const gc = std::min(G, ng - g0);
+          units.insert(units.begin() + nsplit++, make_int4(int(pe), g0, gc, 0));
+          split_rows = std::max(split_rows, Rp * gc);
+          split_sums = std::max(split_sums, 4 * nb * gc);
+        }
+        split_tile = std::max(split_tile, 4 * nb);
+        ++pe;
+        continue;
+      }
       int const G  = std::max(1, std::min(std::min(ng, 27), budget / Rp));
       max_rp       = std::max(max_rp, Rp);
       for (int g0 = 0; g0 < ng; g0 += G)
@@ -1348,6 +1534,8 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
     fac->max_rows = max_rows;
     fac->max_rp   = max_rp;
     fac->nbatches = int(batches.size());
+    fac->nsplit   = nsplit, fac->split_rows = split_rows;
+    fac->split_tile = split_tile, fac->split_sums = split_sums;
     int rc;
     if ((rc = upload(&fac->units, units, bytes)) || (rc = upload(&fac->batches, batches, bytes)) ||
         (rc = upload(&fac->bcells, bcells, bytes)) ||
@@ -1370,10 +1558,12 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
   size_t const wb = sizeof(double) * 2 * size_t(p.rows) * p.tensor;
   ASGK_CUDA(cudaMalloc(&ld->work, wb));
   ASGK_CUDA(cudaStreamCreateWithFlags(&ld->side, cudaStreamNonBlocking));
+  ASGK_CUDA(cudaStreamCreateWithFlags(&ld->side2, cudaStreamNonBlocking));
   for (int q = 0; q < M; q++)
   {
     ASGK_CUDA(cudaEventCreateWithFlags(&ld->fork[q], cudaEventDisableTiming));
     ASGK_CUDA(cudaEventCreateWithFlags(&ld->join[q], cudaEventDisableTiming));
+    ASGK_CUDA(cudaEventCreateWithFlags(&ld->join2[q], cudaEventDisableTiming));
   }
   bytes += int64_t(wb);
   *out = ld.release();
@@ -1410,43 +1600,87 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
   a.st_k = ipow3l(D - 1 - f.k);
   for (int q = 0; q < 3; q++)
     a.st_line[q] = q < M ? ipow3l(D - 1 - ld.line[q]) : 0;
-  bool const both = f.nbatches > 0 && f.nunits > 0;
-  cudaStream_t sb = s;
-  if (both)
-  {
-    sb = ld.side;
+  // the launches of the factor, the first on the caller's stream
+  int const nlarge = f.nunits - f.nsplit;
+  int const parts  = (f.nsplit > 0) + (nlarge > 0) + (f.nbatches > 0);
+  if (parts > 1)
     ASGK_CUDA(cudaEventRecord(ld.fork[KIDX], s));
-    ASGK_CUDA(cudaStreamWaitEvent(sb, ld.fork[KIDX], 0));
-  }
-  if (f.nunits > 0)
+  cudaStream_t const s_split = s;
+  cudaStream_t const s_large = f.nsplit > 0 ? ld.side : s;
+  cudaStream_t const s_small = f.nsplit > 0 && nlarge > 0 ? ld.side2
+                               : (parts > 1 ? ld.side : s);
+  auto fork = [&](cudaStream_t to) -> int {
+    if (to != s)
+      ASGK_CUDA(cudaStreamWaitEvent(to, ld.fork[KIDX], 0));
+    return ASGK_OK;
+  };
+  auto join = [&](cudaStream_t from, cudaEvent_t ev) -> int {
+    if (from != s)
+    {
+      ASGK_CUDA(cudaEventRecord(ev, from));
+      ASGK_CUDA(cudaStreamWaitEvent(s, ev, 0));
+    }
+    return ASGK_OK;
+  };
+  // the (member, group) tables (members x groups <= rows / 3), X, Y and the
+  // matrix tiles (or, in a cluster, the warps' sums)
+  auto shared = [](int rows, size_t tiles) {
+    return ((12 * (size_t(rows) / 3 + 1) + 15) / 16) * 16 +
+           sizeof(R) * (2 * size_t(rows) * NCP + tiles);
+  };
+  if (f.nsplit > 0)
   {
-    // the (member, group) tables (members x groups <= max_rows / 3), X, Y and
-    // the matrix tiles
-    size_t const shm = ((12 * (size_t(f.max_rows) / 3 + 1) + 15) / 16) * 16 +
-                       sizeof(R) * (2 * size_t(f.max_rows) * NCP +
-                                    2 * size_t(kLineTile) * f.max_rp);
-    auto kern        = k_line_factor<R, D, M, KIDX>;
+    size_t const shm =
+        shared(f.split_rows, std::max(2 * size_t(kSplitTile) * f.split_tile,
+                                      size_t(kLineThreads / 32) * f.split_sums * NC));
+    auto kern = k_line_factor<R, D, M, KIDX, kSplit>;
+    ASGK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+    cudaLaunchAttribute cl{};
+    cl.id               = cudaLaunchAttributeClusterDimension;
+    cl.val.clusterDim.x = kSplit;
+    cl.val.clusterDim.y = cl.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = dim3(kSplit * f.nsplit);
+    cfg.blockDim         = dim3(kLineThreads);
+    cfg.dynamicSmemBytes = shm;
+    cfg.stream           = s_split;
+    cfg.attrs            = &cl;
+    cfg.numAttrs         = 1;
+    ASGK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, in64, inR, out64, outR, bj ? 1 : 0, sc, vscale, vc,
+                                 zc, g_gate));
+    count_launch();
+  }
+  if (nlarge > 0)
+  {
+    if (int rc = fork(s_large))
+      return rc;
+    size_t const shm = shared(f.max_rows, 2 * size_t(kLineTile) * f.max_rp);
+    auto kern        = k_line_factor<R, D, M, KIDX, 1>;
     ASGK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(shm)));
-    kern<<<f.nunits, kLineThreads, shm, sb>>>(a, in64, inR, out64, outR, bj ? 1 : 0,
-                                              sc, vscale, vc, zc, g_gate);
+    line_args<R> al = a;
+    al.units += f.nsplit;
+    kern<<<nlarge, kLineThreads, shm, s_large>>>(al, in64, inR, out64, outR, bj ? 1 : 0,
+                                                 sc, vscale, vc, zc, g_gate);
     ASGK_LAUNCHED();
   }
   if (f.nbatches > 0)
   {
+    if (int rc = fork(s_small))
+      return rc;
     size_t const shm = sizeof(R) * size_t(kSmallCells) * ipow3l(D);
     auto kern        = k_line_small<R, D, M, KIDX>;
     ASGK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    int(shm)));
-    kern<<<f.nbatches, kSmallThreads, shm, s>>>(a, f.batches, f.bcells, in64, inR, out64,
-                                                outR, bj ? 1 : 0, sc, vscale, vc, zc, g_gate);
+    kern<<<f.nbatches, kSmallThreads, shm, s_small>>>(a, f.batches, f.bcells, in64, inR, out64,
+                                                      outR, bj ? 1 : 0, sc, vscale, vc, zc, g_gate);
     ASGK_LAUNCHED();
+    if (int rc = join(s_small, ld.join2[KIDX]))
+      return rc;
   }
-  if (both)
-  {
-    ASGK_CUDA(cudaEventRecord(ld.join[KIDX], sb));
-    ASGK_CUDA(cudaStreamWaitEvent(s, ld.join[KIDX], 0));
-  }
+  if (nlarge > 0)
+    if (int rc = join(s_large, ld.join[KIDX]))
+      return rc;
   return ASGK_OK;
 }
 

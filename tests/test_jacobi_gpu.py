@@ -263,3 +263,99 @@ def test_line_jacobi_matches_oracle(cuda, d, L, T):
             its[(name, prec)] = info.iterations
     assert its[("line", "fp64")] <= its[("kron", "fp64")], its
     assert its[("line", "fp32")] <= its[("kron", "fp32")] + 2, its
+
+
+def _line_by_eigh(op, dt, v):
+    """z = M_km^-1 B ... B M_k1^-1 v over the dimensions with a symmetric
+    operator (M_k = I - dt (K_k + the others' cell-diagonal parts), B = I - dt
+    (all their cell-diagonal parts)), pencil by pencil with NumPy's
+    eigendecompositions: grids whose dense pencil systems are too large for
+    oracle.line_jacobi_apply."""
+    d, n = op.d, 3
+    F, n_id = oracle._global_1d_operators(d, op.level, op.terms, op.vA, n)
+    line = oracle.line_dimensions(d, op.level, op.terms, op.vA, n)
+    s = 1.0 - dt * n_id
+    lev, pos = op.table[:, :d].astype(np.int64), op.table[:, d:].astype(np.int64)
+    c1 = np.where(lev == 0, 0, (1 << np.maximum(lev - 1, 0)) + pos)
+    S = {j: np.stack([F[j][n * c:n * c + n, n * c:n * c + n] for c in range(1 << op.level)]) for j in line}
+    eig = {j: np.linalg.eigh(S[j]) for j in line}
+
+    def cellwise(z, j, M):
+        w = z.reshape(op.rows, n ** j, n, -1)
+        return np.einsum("cij,cajb->caib", M[c1[:, j]], w).reshape(z.shape)
+
+    z = v.reshape((op.rows,) + (n,) * d)
+    for i, k in enumerate(line):
+        if i:
+            z = s * z - dt * sum(cellwise(z, j, S[j]) for j in line)
+        others = [j for j in line if j != k]
+        for j in others:
+            z = cellwise(z, j, eig[j][1].transpose(0, 2, 1))
+        den = np.full(z.shape, s)
+        for j in others:
+            den -= dt * eig[j][0][c1[:, j]].reshape((op.rows,) + (1,) * j + (n,) + (1,) * (d - 1 - j))
+        keys = {}
+        for c in range(op.rows):
+            keys.setdefault(tuple(np.delete(c1[c], k)), []).append(c)
+        out, fac = np.empty_like(z), {}
+        for mem in keys.values():
+            mem = np.array(sorted(mem, key=lambda c: c1[c, k]))
+            ids = tuple(c1[mem, k])
+            if ids not in fac:
+                at = np.concatenate([np.arange(n * c, n * c + n) for c in ids])
+                fac[ids] = np.linalg.eigh(F[k][np.ix_(at, at)])
+            th, Q = fac[ids]
+            x = np.moveaxis(z[mem], k + 1, 1).reshape(len(th), -1)
+            dn = np.moveaxis(den[mem], k + 1, 1).reshape(len(th), -1) - dt * th[:, None]
+            y = (Q @ ((Q.T @ x) / dn)).reshape((len(mem), n) + (n,) * (d - 1))
+            out[mem] = np.moveaxis(y, 1, k + 1)
+        z = out
+        for j in others:
+            z = cellwise(z, j, eig[j][1])
+    return z.reshape(-1)
+
+
+@pytest.mark.parametrize("d,L,T", [(2, 4, 2), (2, 6, 2), (2, 7, 2), (3, 7, 3), (4, 5, 4), (4, 6, 4), (4, 7, 4),
+                                   (5, 6, 5), (6, 5, 6), (6, 6, 6)])
+def test_line_jacobi_long_pencils(cuda, d, L, T):
+    """Pencils of 16 to 128 cells, those that a cluster of CTAs shares and
+    those that one CTA takes (1 to 3 line dimensions), against NumPy in FP64.
+    Both sides diagonalise symmetric matrices (errors of a few hundred u, u =
+    2^-53 or 2^-24): 1e-12 as for the short pencils, and in FP32 1e-5."""
+    import asgard_b200 as ab
+    import torch
+    op = ab.SparseGridOperator(d, L, T, kind="advdiff") if d < 6 else None
+    if op is None:          # without the pair list, which this does not need
+        op = ab.SparseGridOperator.__new__(ab.SparseGridOperator)
+        op.d, op.level, op.terms, op.n = d, L, T, 3
+        op.table, op.vA = ab.sparse_grid(d, L), ab.factor_values(d, L, T)
+        op.rows = op.table.shape[0]
+        op.N = op.rows * 3 ** d
+    g = op.kronmult_matrix(mode="global")
+    dt = 1e-3
+    ln = ab.JacobiPreconditioner(g, dt, kind="line")
+    v = np.random.default_rng(d + L).uniform(-1, 1, op.N)
+    expect = _line_by_eigh(op, dt, v)
+    vd = torch.from_numpy(v).cuda()
+    z = torch.zeros_like(vd)
+    for precision, bar in (("fp64", 1e-12), ("fp32", 1e-5)):
+        z.fill_(float("nan"))
+        ln.apply(vd, z, precision=precision)
+        torch.cuda.synchronize()
+        assert rel_err(z.cpu().numpy(), expect) < bar
+    assert np.array_equal(vd.cpu().numpy(), v)
+    # inside recorded cycles the first factor also normalises the basis
+    # vector in place: the same solution as host-driven cycles
+    b = torch.from_numpy(np.random.default_rng(5).uniform(-1, 1, op.N)).cuda()
+    xs = []
+    for graphs in (True, False):
+        old = ab.gmres_settings(graphs=graphs)
+        try:
+            x = torch.zeros_like(b)
+            info = ab.simple_gmres_euler(dt, g, x, b, 50, 300, 1e-10, tol_mode="rel", precision="fp32",
+                                         precond=ln)
+        finally:
+            ab.gmres_settings(**old)
+        assert info.status == 0 and info.true_relres <= 1e-10
+        xs.append(x)
+    assert torch.equal(xs[0], xs[1])
