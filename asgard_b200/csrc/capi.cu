@@ -899,6 +899,7 @@ int record_cycle(gmres_ws &ws, int64_t n, matvec_t const &mat,
     return ASGK_ERR_CUDA;
   cudaStream_t const cs = ws.capture;
   bool const low        = out.key.low_basis;
+  bool const one        = cgs_in_one(n, restart);
   int const S           = std::max(1, std::min(out.key.node_steps, restart));
   int const nodes       = (restart + S - 1) / S;
   cudaGraph_t graph     = nullptr;
@@ -958,21 +959,24 @@ int record_cycle(gmres_ws &ws, int64_t n, matvec_t const &mat,
       }
       else
         rc = mat(1.0, vi, 0.0, w, cs);
-      if (rc == ASGK_OK)
+      givens_args ga;
+      ga.state    = ws.dstate;
+      ga.step     = i;
+      ga.restart  = restart;
+      ga.has_next = (i + 1 == i_end && b + 1 < nodes) ? 1 : 0;
+      ga.next     = ga.has_next ? hs[b + 1] : hs[b];
+      if (rc == ASGK_OK && one)
+        rc = low ? launch_cgs_one_f(ws.Vf, n, k, w, n, ws.h, &ga, cs)
+                 : launch_cgs_one(ws.V, n, k, w, n, ws.h, &ga, cs);
+      else if (rc == ASGK_OK)
+      {
         rc = low ? launch_multidot_hf(ws.Vf, n, k, w, n, ws.part, ws.tickets + 2, ws.h, cs)
                  : launch_multidot_h(ws.V, n, k, w, n, ws.part, ws.tickets + 2, ws.h, cs);
-      if (rc == ASGK_OK)
-      {
-        givens_args ga;
-        ga.state    = ws.dstate;
-        ga.step     = i;
-        ga.restart  = restart;
-        ga.has_next = (i + 1 == i_end && b + 1 < nodes) ? 1 : 0;
-        ga.next     = ga.has_next ? hs[b + 1] : hs[b];
-        rc = low ? launch_update_norm_hf(ws.Vf, n, k, ws.h, w, n, ws.part, ws.tickets,
-                                         ws.h + k, cs, &ga)
-                 : launch_update_norm_h(ws.V, n, k, ws.h, w, n, ws.part, ws.tickets,
-                                        ws.h + k, cs, &ga);
+        if (rc == ASGK_OK)
+          rc = low ? launch_update_norm_hf(ws.Vf, n, k, ws.h, w, n, ws.part, ws.tickets,
+                                           ws.h + k, cs, &ga)
+                   : launch_update_norm_h(ws.V, n, k, ws.h, w, n, ws.part, ws.tickets,
+                                          ws.h + k, cs, &ga);
       }
       // without a preconditioner to fold it into, w is normalised here, with
       // its FP32 copy when there is one.  The last step's w is never read
@@ -1154,16 +1158,25 @@ int gmres_core(gmres_ws &ws, int64_t n, matvec_t const &mat,
       ++st.total;
       ++st.matvecs;
       int const k = inner + 1;
-      if (int rc = low ? launch_multidot_hf(ws.Vf, n, k, w, n, ws.part,
-                                            ws.tickets + 2, ws.h, s)
-                       : launch_multidot_h(ws.V, n, k, w, n, ws.part,
-                                           ws.tickets + 2, ws.h, s))
-        return rc;
-      if (int rc = low ? launch_update_norm_hf(ws.Vf, n, k, ws.h, w, n, ws.part,
-                                               ws.tickets, ws.h + k, s)
-                       : launch_update_norm_h(ws.V, n, k, ws.h, w, n, ws.part,
-                                              ws.tickets, ws.h + k, s))
-        return rc;
+      if (cgs_in_one(n, restart))
+      {
+        if (int rc = low ? launch_cgs_one_f(ws.Vf, n, k, w, n, ws.h, nullptr, s)
+                         : launch_cgs_one(ws.V, n, k, w, n, ws.h, nullptr, s))
+          return rc;
+      }
+      else
+      {
+        if (int rc = low ? launch_multidot_hf(ws.Vf, n, k, w, n, ws.part,
+                                              ws.tickets + 2, ws.h, s)
+                         : launch_multidot_h(ws.V, n, k, w, n, ws.part,
+                                             ws.tickets + 2, ws.h, s))
+          return rc;
+        if (int rc = low ? launch_update_norm_hf(ws.Vf, n, k, ws.h, w, n, ws.part,
+                                                 ws.tickets, ws.h + k, s)
+                         : launch_update_norm_h(ws.V, n, k, ws.h, w, n, ws.part,
+                                                ws.tickets, ws.h + k, s))
+          return rc;
+      }
       if (int rc = read_small(ws.hh, ws.hh_dev, ws.h, k + 1, s))
         return rc;
       ASGK_CUDA(cudaStreamSynchronize(s));

@@ -8,6 +8,7 @@ namespace asgk
 // before it (remote ones too) before those after it
 __device__ __forceinline__ void cluster_sync()
 {
+  __syncwarp(); // the barrier's aligned form is taken by whole warps
   asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
                "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -313,6 +313,13 @@ int launch_update_norm_hf(const float *V, int64_t ldv, int k, const double *h,
                           double *w, int64_t n, double *part, unsigned *ticket,
                           double *out, cudaStream_t s,
                           givens_args const *ga = nullptr);
+// both passes and the Givens update of a short basis in one launch
+// (cgs_in_one): h[0..k) = V^T w, w -= V h, h[k] = ||w||^2
+bool cgs_in_one(int64_t n, int restart);
+int launch_cgs_one(const double *V, int64_t ldv, int k, double *w, int64_t n, double *h,
+                   givens_args const *ga, cudaStream_t s);
+int launch_cgs_one_f(const float *V, int64_t ldv, int k, double *w, int64_t n, double *h,
+                     givens_args const *ga, cudaStream_t s);
 // w *= f, vf = FP32(w); f = state[1] when state is set, else scale
 int launch_store_basis(double *w, float *vf, int64_t n, const double *state,
                        double scale, cudaStream_t s);

@@ -5,6 +5,7 @@
 // the classical Gram-Schmidt step reads the Krylov basis exactly twice (one
 // multi-dot pass, one fused "w -= V h" + norm pass) and every reduction is
 // deterministic: fixed grid, per-block partial sums, then an ordered sum.
+#include "cluster.cuh"
 #include "gmres_device.cuh"
 
 #include <algorithm>
@@ -179,6 +180,14 @@ __global__ void k_reduce_parts(const double *__restrict__ part, int blocks,
     out[j] = v[0];
 }
 
+// The last of a thread's rows first, first + step, ... below n (negative:
+// none).  The update passes go through the rows backwards: the multi-dot
+// before them went forwards, so the basis rows it read last are still in L2.
+__device__ __forceinline__ int64_t last_row(int64_t first, int64_t step, int64_t n)
+{
+  return first >= n ? -1 : first + (n - 1 - first) / step * step;
+}
+
 // sum_j V[r, j] hs[j], four chains by column mod 4
 __device__ __forceinline__ double dot_row(const double *__restrict__ V,
                                           int64_t ldv, int k, int64_t r,
@@ -261,7 +270,8 @@ __global__ void __launch_bounds__(kUpdateThreads)
   const T *Vu        = reinterpret_cast<const T *>(V);
   T *wu              = reinterpret_cast<T *>(w);
   double v[1]        = {0.0};
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < nu; r += step)
+  for (int64_t r = last_row(blockIdx.x * int64_t(blockDim.x) + threadIdx.x, step, nu); r >= 0;
+       r -= step)
   {
     double s[VEC];
     dot_rows<VEC>(Vu, ldv / VEC, k, r, hs, s);
@@ -439,9 +449,8 @@ __global__ void __launch_bounds__(kThreads)
   using T = typename vload<VEC>::T;
   __shared__ double sh[kDotCols * 32];
   int64_t const nu    = n / VEC;
-  int64_t const chunk = (nu + gridDim.x - 1) / gridDim.x;
-  int64_t const beg   = blockIdx.x * chunk;
-  int64_t const end   = min(nu, beg + chunk);
+  int64_t const step  = int64_t(gridDim.x) * blockDim.x;
+  int64_t const beg   = blockIdx.x * int64_t(blockDim.x);
   int const j0        = blockIdx.y * kDotCols;
   int const nj        = min(kDotCols, k - j0);
   int64_t const ldu   = ldv / VEC;
@@ -451,7 +460,7 @@ __global__ void __launch_bounds__(kThreads)
     a[j] = 0.0;
   const T *Vj = reinterpret_cast<const T *>(V + int64_t(j0) * ldv);
   const T *wu = reinterpret_cast<const T *>(w);
-  for (int64_t r = beg + threadIdx.x; r < end; r += blockDim.x)
+  for (int64_t r = beg + threadIdx.x; r < nu; r += step)
   {
     T const wr = wu[r];
 #pragma unroll
@@ -496,14 +505,13 @@ __global__ void __launch_bounds__(kThreads)
     hs[j] = h[j];
   __syncthreads();
   int64_t const nu    = n / VEC;
-  int64_t const chunk = (nu + gridDim.x - 1) / gridDim.x;
-  int64_t const beg   = blockIdx.x * chunk;
-  int64_t const end   = min(nu, beg + chunk);
+  int64_t const step  = int64_t(gridDim.x) * blockDim.x;
+  int64_t const beg   = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   int64_t const ldu   = ldv / VEC;
   const T *Vu = reinterpret_cast<const T *>(V);
   T *wu       = reinterpret_cast<T *>(w);
   double v[1] = {0.0};
-  for (int64_t r = beg + threadIdx.x; r < end; r += blockDim.x)
+  for (int64_t r = last_row(beg, step, nu); r >= 0; r -= step)
   {
     if constexpr (VEC == 1)
     {
@@ -634,9 +642,8 @@ __global__ void __launch_bounds__(kThreads)
   using T = typename fload<VEC>::T;
   __shared__ double sh[kDotCols * 32];
   int64_t const nu    = n / VEC;
-  int64_t const chunk = (nu + gridDim.x - 1) / gridDim.x;
-  int64_t const beg   = blockIdx.x * chunk;
-  int64_t const end   = min(nu, beg + chunk);
+  int64_t const step  = int64_t(gridDim.x) * blockDim.x;
+  int64_t const beg   = blockIdx.x * int64_t(blockDim.x);
   int const j0        = blockIdx.y * kDotCols;
   int const nj        = min(kDotCols, k - j0);
   int64_t const ldu   = ldv / VEC;
@@ -645,7 +652,7 @@ __global__ void __launch_bounds__(kThreads)
   for (int j = 0; j < kDotCols; j++)
     a[j] = 0.0;
   const T *Vj = reinterpret_cast<const T *>(V + int64_t(j0) * ldv);
-  for (int64_t r = beg + threadIdx.x; r < end; r += blockDim.x)
+  for (int64_t r = beg + threadIdx.x; r < nu; r += step)
   {
     double wr[VEC];
     load_rows<VEC>(w, r, wr);
@@ -689,13 +696,12 @@ __global__ void __launch_bounds__(kThreads)
     hs[j] = h[j];
   __syncthreads();
   int64_t const nu    = n / VEC;
-  int64_t const chunk = (nu + gridDim.x - 1) / gridDim.x;
-  int64_t const beg   = blockIdx.x * chunk;
-  int64_t const end   = min(nu, beg + chunk);
+  int64_t const step  = int64_t(gridDim.x) * blockDim.x;
+  int64_t const beg   = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   int64_t const ldu   = ldv / VEC;
   const T *Vu         = reinterpret_cast<const T *>(V);
   double v[1]         = {0.0};
-  for (int64_t r = beg + threadIdx.x; r < end; r += blockDim.x)
+  for (int64_t r = last_row(beg, step, nu); r >= 0; r -= step)
   {
     // eight basis loads in flight, four partial sums per row
     double acc[4][VEC];
@@ -761,6 +767,115 @@ __global__ void k_store_basis(double *__restrict__ w, float *__restrict__ vf,
     else
       reinterpret_cast<float2 *>(vf)[r] = make_float2(float(x[0]), float(x[1]));
   }
+}
+
+// ---- a whole Gram-Schmidt step of a short basis in one launch -----------
+//
+// For vectors of up to kStepRows values the two passes above are a few
+// microseconds of launch and reduction latency each.  One cluster of kStepCtas CTAs does the step: every CTA
+// holds its rows of w in shared memory, sends its partial projections (a
+// warp per column) and its part of ||w||^2 to the others' shared memory, and
+// adds them in rank order, so the sums have a fixed order.  h[0..k) and
+// h[k] = ||w||^2 as the passes leave them; ga as in k_update_norm_h.  Four
+// plain GMRES time steps on 2304 values: 15.5 -> 14.6 ms; two on 7344 took
+// 8.07 ms with the passes and 8.51 in one launch, so the line lies between.
+constexpr int kStepCtas      = 8;
+constexpr int kStepThreads   = 512;
+constexpr int64_t kStepRows  = 4096;
+constexpr int kStepRestart   = 512; // 8 partial sums per column in shared memory
+template<typename BT>
+__global__ void __launch_bounds__(kStepThreads)
+    k_cgs_cluster(const BT *__restrict__ V, int64_t ldv, int k, double *__restrict__ w, int n,
+                  double *__restrict__ h, givens_args ga, const double *__restrict__ gate)
+{
+  if (gate_closed(gate))
+    return;
+  extern __shared__ double step_smem[];
+  __shared__ double sh[32];
+  int const rank = cluster_rank();
+  int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int const rows = (n + kStepCtas - 1) / kStepCtas;
+  int const beg  = min(n, rank * rows), cnt = min(n, beg + rows) - beg;
+  double *ws     = step_smem;           // the CTA's rows of w
+  double *part   = ws + rows;           // [kStepCtas][k + 1]
+  double *hs     = part + kStepCtas * (k + 1);
+  for (int r = threadIdx.x; r < cnt; r += kStepThreads)
+    ws[r] = w[beg + r];
+  cluster_sync(); // ws is complete, and every CTA runs
+  for (int j = warp; j < k; j += kStepThreads / 32)
+  {
+    const BT *v = V + int64_t(j) * ldv + beg;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int r = lane;
+    for (; r + 96 < cnt; r += 128)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        a[q] = fma(double(v[r + 32 * q]), ws[r + 32 * q], a[q]);
+    for (; r < cnt; r += 32)
+      a[0] = fma(double(v[r]), ws[r], a[0]);
+    double s = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0)
+      put_all<kStepCtas>(part + rank * (k + 1) + j, s);
+  }
+  cluster_sync();
+  for (int j = threadIdx.x; j < k; j += kStepThreads)
+  {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kStepCtas; c++)
+      s += part[c * (k + 1) + j];
+    hs[j] = s;
+    if (rank == 0)
+      h[j] = s;
+  }
+  __syncthreads();
+  double v2[1] = {0.0};
+  for (int r = threadIdx.x; r < cnt; r += kStepThreads)
+  {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    const BT *v = V + beg + r;
+    int j = 0;
+    for (; j + 8 <= k; j += 8)
+    {
+      BT u[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        u[q] = v[(j + q) * ldv];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        a[q & 3] = fma(double(u[q]), hs[j + q], a[q & 3]);
+    }
+    for (; j < k; j++)
+      a[j & 3] = fma(double(v[j * ldv]), hs[j], a[j & 3]);
+    double const x = ws[r] - ((a[0] + a[1]) + (a[2] + a[3]));
+    w[beg + r]     = x;
+    v2[0] += x * x;
+  }
+  block_sum<1>(v2, sh);
+  if (threadIdx.x == 0)
+    put_all<kStepCtas>(part + rank * (k + 1) + k, v2[0]);
+  cluster_sync(); // the last remote store: CTAs may end at any time from here
+  double nrm2 = 0.0;
+#pragma unroll
+  for (int c = 0; c < kStepCtas; c++)
+    nrm2 += part[c * (k + 1) + k];
+  if (rank != 0)
+    return;
+  if (threadIdx.x == 0)
+    h[k] = nrm2;
+  if (ga.state == nullptr)
+    return;
+  double *csn    = hs + k;                     // cosines, sines: 2*(restart+1)
+  double *coeffs = csn + 2 * (ga.restart + 1); // k
+  const double *cs_g = ga.state + kStateHead + ga.restart + 1;
+  for (int j = threadIdx.x; j < 2 * (ga.restart + 1); j += kStepThreads)
+    csn[j] = (j % (ga.restart + 1) < ga.step) ? cs_g[j] : 0.0;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    givens_step(ga, hs, nrm2, coeffs, csn);
 }
 
 // *out = ||x||^2
@@ -893,6 +1008,46 @@ int launch_update_norm_hf(const float *V, int64_t ldv, int k, const double *h,
                                                 g_gate);
   ASGK_LAUNCHED();
   return ASGK_OK;
+}
+
+bool cgs_in_one(int64_t n, int restart) { return n <= kStepRows && restart <= kStepRestart; }
+
+template<typename BT>
+static int cgs_cluster(const BT *V, int64_t ldv, int k, double *w, int64_t n, double *h,
+                       givens_args const *ga, cudaStream_t s)
+{
+  givens_args const a = ga ? *ga : givens_args{};
+  int64_t const rows  = (n + kStepCtas - 1) / kStepCtas;
+  size_t const shm    = sizeof(double) * (rows + int64_t(kStepCtas) * (k + 1) + 2 * int64_t(k) +
+                                       2 * int64_t(a.restart + 1));
+  ASGK_CUDA(cudaFuncSetAttribute(k_cgs_cluster<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(shm)));
+  cudaLaunchAttribute cl{};
+  cl.id               = cudaLaunchAttributeClusterDimension;
+  cl.val.clusterDim.x = kStepCtas;
+  cl.val.clusterDim.y = cl.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim          = dim3(kStepCtas);
+  cfg.blockDim         = dim3(kStepThreads);
+  cfg.dynamicSmemBytes = shm;
+  cfg.stream           = s;
+  cfg.attrs            = &cl;
+  cfg.numAttrs         = 1;
+  ASGK_CUDA(cudaLaunchKernelEx(&cfg, k_cgs_cluster<BT>, V, ldv, k, w, int(n), h, a, g_gate));
+  count_launch();
+  return ASGK_OK;
+}
+
+int launch_cgs_one(const double *V, int64_t ldv, int k, double *w, int64_t n, double *h,
+                   givens_args const *ga, cudaStream_t s)
+{
+  return cgs_cluster(V, ldv, k, w, n, h, ga, s);
+}
+
+int launch_cgs_one_f(const float *V, int64_t ldv, int k, double *w, int64_t n, double *h,
+                     givens_args const *ga, cudaStream_t s)
+{
+  return cgs_cluster(V, ldv, k, w, n, h, ga, s);
 }
 
 int launch_store_basis(double *w, float *vf, int64_t n, const double *state,

@@ -16,7 +16,7 @@ dimensions, chained (the learned correction on top of it is trained and kept
 only if its validation solve gains), FP32 operator inside FP64 iterative
 refinement.  Timed beside it: the plain
 baseline -- FP64 GMRES with the connected-pair FP64 kronmult (one solve by
-default: about four minutes at d=6) -- and, at d <= 4, the same method on the
+default) -- and, at d <= 4, the same method on the
 connected-pair operator.  Inputs are resident in HBM when the timed region
 starts; at d=6 every vector (94 MB) and the plain baseline's pair list
 (6.3 GB) are larger than L2, at d=4 the method's working set is L2-sized by
@@ -63,7 +63,6 @@ TOL = 1e-10
 # each workload's operator kernels, from one ncu capture of that kernel on
 # that workload; None where no capture was taken.
 KERNEL_TRAFFIC = {
-    ("pairs", "d4"): 254_243_328 + 4_232_704,
     ("global", "d4"): 3_930_368,
     ("global", "d6"): 71_265_792 + 54_134_016,
 }
@@ -77,7 +76,7 @@ def parse():
     ap.add_argument("--impl", default="mine", choices=["mine", "reference"])
     ap.add_argument("--workload", default="d6", choices=sorted(WORKLOADS))
     ap.add_argument("--plain-steps", type=int, default=1,
-                    help="timed plain FP64 solves (about 250 s each at d=6)")
+                    help="timed plain FP64 solves")
     ap.add_argument("--pair-method-steps", type=int, default=None,
                     help="timed solves of the method on the connected-pair "
                          "operator (default 2 at d <= 4, 0 above)")
@@ -692,9 +691,9 @@ def precision_forms(op, gmat, method, dt, B, steps, solve, plain_value):
 
 def rooflines(ab, op, mat, gmat, method, dt, workload, xs):
     """Average launch durations by CUDA events on the launching stream: the
-    method's operator kernel (global form, algorithmic bytes against the
-    measured HBM bandwidth) and the plain baseline's connected-pair kernel
-    (algorithmic flops against the live-measured FP64 FMA peak)."""
+    method's operator kernel (global form) and the plain baseline's
+    connected-pair apply, algorithmic bytes against the measured HBM
+    bandwidth.  pair_flops: what the pairs one by one would take."""
     import torch
     d, N = op.d, op.N
     ys = torch.zeros_like(xs)
@@ -712,26 +711,21 @@ def rooflines(ab, op, mat, gmat, method, dt, workload, xs):
         torch.cuda.synchronize()
         return a0.elapsed_time(a1) / 1e3 / reps
 
-    preps = 5 if d <= 4 else 2
+    preps = 5
     t64 = time_apply(mat, "fp64", preps)
     t32 = time_apply(mat, "fp32", preps)
-    fp64_peak = ab._lib.C.c_double()
-    ab.lib.asgk_measure_fma_peak(0, ab._lib.C.byref(fp64_peak))
-    fp32_peak = ab._lib.C.c_double()
-    ab.lib.asgk_measure_fma_peak(1, ab._lib.C.byref(fp32_peak))
-    pair_kernel = (f"kron3_staged<d={d}, fp64> (+ x repack)" if d in (3, 4)
-                   else f"kron3_rows<d={d}, fp64>")
-    pair_roof = {"bound": "fp64", "kernel": pair_kernel,
-                 "achieved": flops / t64 / 1e12, "peak": fp64_peak.value,
-                 "peak_source": "measured live (FMA chain kernel)",
-                 "unit": "TFLOP/s", "frac": flops / t64 / 1e12 / fp64_peak.value,
+    # the pair list is a whole grid's, so its apply is the tree of 1D passes:
+    # algorithmic bytes are x read once, y written and the factors read once
+    pbytes = 16 * N + 8 * len(op.vA)
+    phbm, psrc = _measured_hbm_gbs()
+    pair_roof = {"bound": "hbm", "kernel": f"k_sweep<d={d}, fp64> (one apply of the tree)",
+                 "achieved": pbytes / t64 / 1e9, "peak": phbm, "peak_source": psrc,
+                 "unit": "GB/s", "frac": pbytes / t64 / 1e9 / phbm,
                  "traffic": KERNEL_TRAFFIC.get(("pairs", workload)),
-                 "traffic_source": "ncu dram__bytes_read+write, one launch",
-                 "ms_per_launch": t64 * 1e3, "flops_per_launch": flops,
-                 "fp32_kernel": {"ms_per_launch": t32 * 1e3,
-                                 "achieved": flops / t32 / 1e12,
-                                 "peak": fp32_peak.value,
-                                 "frac": flops / t32 / 1e12 / fp32_peak.value}}
+                 "traffic_source": "not captured",
+                 "ms_per_launch": t64 * 1e3, "bytes_per_launch": pbytes,
+                 "pair_flops": flops,
+                 "fp32_kernel": {"ms_per_launch": t32 * 1e3}}
     if gmat is None:
         return pair_roof
     # the method's operator kernel: algorithmic bytes per launch are x read

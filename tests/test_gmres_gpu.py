@@ -364,3 +364,38 @@ def test_steps_per_node_on_every_operator_form(cuda, plan):
             got.append((info.iterations, x))
         assert len({it for it, _ in got}) == 1 and got[0][0] > 3
         assert all(torch.equal(got[0][1], x) for _, x in got[1:])
+
+
+@pytest.mark.parametrize("cells", [1, 2, 455, 456])
+def test_solves_beside_the_one_launch_step(cuda, cells):
+    """Vectors from shorter than a cluster has CTAs to both sides of the
+    longest that take the Gram-Schmidt step in one launch (4096 values): the
+    solution of a block-diagonal system, FP64 and FP32, recorded and
+    host-driven cycles bit for bit."""
+    import asgard_b200 as ab
+    import torch
+    d, n = 2, 3
+    rng = np.random.default_rng(cells)
+    A = rng.uniform(-1, 1, (2, n * n))
+    iA = np.tile(np.array([0, n * n], np.int32), cells)     # every cell with itself
+    mat = ab.kronmult_matrix.from_csr(d, n, cells, cells, 1, np.arange(cells + 1), np.arange(cells),
+                                      iA, A.ravel())
+    K = np.kron(A[0].reshape(n, n, order="F"), A[1].reshape(n, n, order="F"))
+    b = rng.uniform(-1, 1, (cells, n * n))
+    dt = 0.05
+    expect = np.linalg.solve(np.eye(n * n) - dt * K, b.T).T.ravel()
+    for precision in ("fp64", "fp32"):
+        got = []
+        for graphs in (True, False):
+            old = ab.gmres_settings(graphs=graphs)
+            try:
+                x = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+                info = ab.simple_gmres_euler(dt, mat, x, torch.from_numpy(b.ravel()).cuda(), 9, 50, 1e-12,
+                                             tol_mode="rel", precision=precision)
+            finally:
+                ab.gmres_settings(**old)
+            assert info.status == 0
+            got.append(x)
+        assert torch.equal(got[0], got[1])
+        # ||x - exact|| <= ||(I - dt K)^-1|| ||r||, and ||dt K|| < 1/2 here
+        assert rel_err(got[0].cpu().numpy(), expect) < 1e-11
