@@ -135,7 +135,7 @@ class kronmult_matrix:
         """Global Kronecker form of the sparse grid's operator: the element
         table (cells x 2d) and vA in the per-1D-connection layout.  Terms
         acting in one dimension are applied in one pass, terms acting in
-        several as the reference's chains of upper/lower 1D passes."""
+        several as a tree of upper, whole and lower 1D passes."""
         tb = _host(table, np.int32)
         vA = _host(vA, np.float64)
         cells = tb.shape[0]

@@ -191,7 +191,7 @@ class SparseGridOperator:
         """mode "pairs": the connected-pair kronmult (expanded: the
         reference's iA offsets instead of connection indices); "global": the
         global Kronecker form (one pass per term acting in one dimension,
-        upper/lower chains for terms acting in several); "dense":
+        a tree of 1D passes for terms acting in several); "dense":
         the reference's dense form (every cell pair, full 1D operators)."""
         from .kronmult import kronmult_matrix
         if mode == "global":

@@ -149,11 +149,13 @@ int asgk_plan_kind(const asgk_plan *plan);
  * differ in at most one dimension.  A term that is the identity
  * (self-connection blocks I, all others 0) in all dimensions but one is
  * applied in one pass with the others; a term acting in m >= 2 dimensions
- * as the reference does it: 2^(m-1) chains of m 1D passes over the upper or
- * lower parts of its 1D operators (its permutes), summed.  n = 3 only.  The
+ * as a tree of 1D passes over the upper, whole and lower parts of its 1D
+ * operators, the reference's 2^(m-1) chains of m passes with their common
+ * beginnings and ends done once.  n = 3 only.  The
  * plan works with asgk_apply / asgk_apply_euler / the GMRES and Jacobi
  * entries like any other; asgk_plan_info's num_batch reports the neighbour
- * entries one apply visits and flops 2 * n^(d+1) per entry.
+ * entries of the terms' passes (the separate chains' for those that act in
+ * several dimensions) and flops 2 * n^(d+1) per entry.
  * asgk_plan_update_values keeps the dimensions each term acts in
  * (ASGK_ERR_INVALID if they change). */
 int asgk_plan_create_global(asgk_plan **plan, int d, int n, int level,
