@@ -63,6 +63,29 @@ __device__ __forceinline__ bool gate_closed(const double *gate)
     ::asgk::count_launch();                                                    \
   } while (0)
 
+#ifdef __CUDACC__
+// The dynamic shared memory that a kernel launched at several sizes is
+// allowed: all that a block can have.  The limit (cudaFuncSetAttribute)
+// belongs to the function, for every thread of the process, and a launch
+// above it fails, so it is the same at every launch; one set to the launch's
+// own size would refuse a larger launch that another thread is about to make.
+inline int shared_ceiling(const void *kern)
+{
+  cudaFuncAttributes a{};
+  if (cudaFuncGetAttributes(&a, kern) != cudaSuccess)
+  {
+    cudaGetLastError();
+    a.sharedSizeBytes = 1024; // more static arrays than any kernel here has
+  }
+  return 227 * 1024 - int(a.sharedSizeBytes);
+}
+template<typename K>
+cudaError_t allow_shared(K *kern, int ceiling)
+{
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ceiling);
+}
+#endif
+
 // Entries of a global-form neighbour list handled by one CTA (4 warps for
 // tensors of up to 81 entries, 8 above).  Measured at d=3/4, level 7: 64
 // beats 16, 32 and 128.

@@ -808,9 +808,8 @@ int jacobi_build(plan_data const &p, double dt, int kind, jacobi_data &jd)
     ASGK_CUDA(cudaMalloc(&jd.M16, sizeof(__half) * bh));
     jd.device_bytes = int64_t(b * sizeof(double) + bh * sizeof(__half));
     size_t const shm = sizeof(double) * size_t(ts) * 2 * ts;
-    ASGK_CUDA(cudaFuncSetAttribute(k_block_jacobi,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(shm)));
+    static int const most = shared_ceiling(reinterpret_cast<const void *>(k_block_jacobi));
+    ASGK_CUDA(allow_shared(k_block_jacobi, most));
     k_block_jacobi<<<p.rows, 256, shm>>>(p.rows, p.d, p.n, ts, p.terms, p.mode,
                                          p.row_ptr, p.col, p.idx, vA, dt,
                                          jd.M64, jd.M16, jd.ps16, err);

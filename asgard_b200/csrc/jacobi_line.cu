@@ -1634,7 +1634,8 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
         shared(f.split_rows, std::max(2 * size_t(kSplitTile) * f.split_tile,
                                       size_t(kLineThreads / 32) * f.split_sums * NC));
     auto kern = k_line_factor<R, D, M, KIDX, kSplit>;
-    ASGK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+    static int const most = shared_ceiling(reinterpret_cast<const void *>(kern));
+    ASGK_CUDA(allow_shared(kern, most));
     cudaLaunchAttribute cl{};
     cl.id               = cudaLaunchAttributeClusterDimension;
     cl.val.clusterDim.x = kSplit;
@@ -1656,8 +1657,8 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
       return rc;
     size_t const shm = shared(f.max_rows, 2 * size_t(kLineTile) * f.max_rp);
     auto kern        = k_line_factor<R, D, M, KIDX, 1>;
-    ASGK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   int(shm)));
+    static int const most = shared_ceiling(reinterpret_cast<const void *>(kern));
+    ASGK_CUDA(allow_shared(kern, most));
     line_args<R> al = a;
     al.units += f.nsplit;
     kern<<<nlarge, kLineThreads, shm, s_large>>>(al, in64, inR, out64, outR, bj ? 1 : 0,

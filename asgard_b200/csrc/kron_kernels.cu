@@ -430,8 +430,8 @@ int launch_generic(plan_data const &p, const TC *vA, double alpha, const TX *x,
   if (shm > 200 * 1024)
     return ASGK_ERR_UNSUPPORTED;
   auto kern = kron_generic_rows<TC, TX, TY, EULER>;
-  ASGK_CUDA(cudaFuncSetAttribute(
-      kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm)));
+  static int const most = shared_ceiling(reinterpret_cast<const void *>(kern));
+  ASGK_CUDA(allow_shared(kern, most));
   int threads = 32;
   while (threads < p.tensor && threads < 256)
     threads *= 2;

@@ -1020,8 +1020,9 @@ static int cgs_cluster(const BT *V, int64_t ldv, int k, double *w, int64_t n, do
   int64_t const rows  = (n + kStepCtas - 1) / kStepCtas;
   size_t const shm    = sizeof(double) * (rows + int64_t(kStepCtas) * (k + 1) + 2 * int64_t(k) +
                                        2 * int64_t(a.restart + 1));
-  ASGK_CUDA(cudaFuncSetAttribute(k_cgs_cluster<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(shm)));
+  static int const most =
+      shared_ceiling(reinterpret_cast<const void *>(k_cgs_cluster<BT>));
+  ASGK_CUDA(allow_shared(k_cgs_cluster<BT>, most));
   cudaLaunchAttribute cl{};
   cl.id               = cudaLaunchAttributeClusterDimension;
   cl.val.clusterDim.x = kStepCtas;
