@@ -2410,6 +2410,9 @@ int gmres_euler_impl(asgk_plan *plan, double dt, double *x, const double *b,
   if (!(tol > 0))
     tol = 1e-12; // src/solver.cpp:165-166 default for double
   cudaStream_t s = as_stream(stream);
+  sweep_turn turn(p.sweep);
+  if (int rc = turn.wait(s))
+    return rc;
   auto *ex       = extras_of(plan, true);
   gmres_ws &ws   = ex->ws;
 

@@ -285,8 +285,24 @@ inline bool sweep_pays(int d, int64_t products, bool fp32)
   int64_t const least = d <= 3 ? 400000 : (d == 4 ? 262144 : 65536);
   return products >= (fp32 ? least * 3 / 2 : least);
 }
-int launch_sweep(plan_data const &p, sweep_data const &w, int precision, double alpha,
-                 const void *x, bool f32, double beta, void *y, double ex, cudaStream_t s);
+int launch_sweep(plan_data const &p, sweep_data &w, int precision, double alpha, const void *x,
+                 bool f32, double beta, void *y, double ex, cudaStream_t s);
+// A turn with the tree's vectors (w null: none are held): no other thread
+// enqueues an apply meanwhile, and what s runs after wait comes after the
+// applies enqueued before.  A solve holds one, as its recorded cycles use the
+// vectors without asking.
+class sweep_turn
+{
+public:
+  explicit sweep_turn(sweep_data *w);
+  ~sweep_turn();
+  sweep_turn(sweep_turn const &) = delete;
+  sweep_turn &operator=(sweep_turn const &) = delete;
+  int wait(cudaStream_t s);
+
+private:
+  sweep_data *w_;
+};
 
 // kron_tc.cu: the tensor-core form (tcgen05, BF16 operands, FP32 TMEM
 // accumulators) of a global plan whose terms act in one dimension each.

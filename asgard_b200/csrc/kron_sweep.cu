@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <type_traits>
@@ -60,6 +61,11 @@ struct sweep_data
   int4 *jobs  = nullptr;
   int *last   = nullptr; // [nresults] the vectors whose sum is the product
   double *work = nullptr;
+  // Whose turn with work it is: one thread enqueues at a time, and an apply
+  // on any stream waits for the one before it (done, once used is set).
+  std::recursive_mutex turn;
+  cudaEvent_t done = nullptr;
+  bool used        = false;
   int nresults = 0;
   sweep_units su[6][3];
   std::vector<sweep_launch> launches;
@@ -786,6 +792,8 @@ void sweep_free(sweep_data *w)
   cudaFree(w->jobs);
   cudaFree(w->last);
   cudaFree(w->work);
+  if (w->done)
+    cudaEventDestroy(w->done);
   delete w;
 }
 
@@ -869,15 +877,16 @@ int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
     w->work = nullptr;
     return ASGK_ERR_ALLOC;
   }
+  ASGK_CUDA(cudaEventCreateWithFlags(&w->done, cudaEventDisableTiming));
   bytes += held + int64_t(b);
   *out = w.release();
   return ASGK_OK;
 }
 
-// y = beta y + alpha (sum of the terms) x + ex x, the vectors of FP32
-// (x_f32: arithmetic FP32) or FP64
-int launch_sweep(plan_data const &p, sweep_data const &w, int precision, double alpha,
-                 const void *x, bool f32, double beta, void *y, double ex, cudaStream_t s)
+namespace
+{
+int launch_tree(plan_data const &p, sweep_data const &w, int precision, double alpha,
+                const void *x, bool f32, double beta, void *y, double ex, cudaStream_t s)
 {
   if (f32)
     return launch_t<float, float, float>(w, p.vP32, p.terms, alpha, static_cast<const float *>(x),
@@ -889,6 +898,44 @@ int launch_sweep(plan_data const &p, sweep_data const &w, int precision, double 
   if (precision == ASGK_FP32)
     return launch_t<float, double, double>(w, p.vP32, p.terms, alpha, xd, beta, yd, ex, s);
   return ASGK_ERR_UNSUPPORTED;
+}
+} // namespace
+
+sweep_turn::sweep_turn(sweep_data *w) : w_(w)
+{
+  if (w_)
+    w_->turn.lock();
+}
+sweep_turn::~sweep_turn()
+{
+  if (w_)
+    w_->turn.unlock();
+}
+int sweep_turn::wait(cudaStream_t s)
+{
+  if (w_ && w_->used)
+    ASGK_CUDA(cudaStreamWaitEvent(s, w_->done, 0));
+  return ASGK_OK;
+}
+
+// y = beta y + alpha (sum of the terms) x + ex x, the vectors of FP32
+// (x_f32: arithmetic FP32) or FP64
+int launch_sweep(plan_data const &p, sweep_data &w, int precision, double alpha, const void *x,
+                 bool f32, double beta, void *y, double ex, cudaStream_t s)
+{
+  // what is recorded runs where the graph is launched
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+  if (!g_recording)
+    ASGK_CUDA(cudaStreamIsCapturing(s, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+    return launch_tree(p, w, precision, alpha, x, f32, beta, y, ex, s);
+  sweep_turn turn(&w);
+  if (int rc = turn.wait(s))
+    return rc;
+  int const rc = launch_tree(p, w, precision, alpha, x, f32, beta, y, ex, s);
+  ASGK_CUDA(cudaEventRecord(w.done, s));
+  w.used = true;
+  return rc;
 }
 
 } // namespace asgk

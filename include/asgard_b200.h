@@ -7,7 +7,13 @@
  * A plan is not re-entrant: one call at a time per plan, as with the
  * reference's kronmult_matrix::apply, which is documented "not thread-safe"
  * (src/asgard_kronmult_matrix.hpp:336).  Calls are stream-ordered on the
- * stream argument (0 = the legacy default stream).
+ * stream argument (0 = the legacy default stream).  An apply may use work
+ * vectors that the plan holds: order the calls of one plan on different
+ * streams with events.  (Pair plans at d = 2, 5, 6 and with FP32 vectors need
+ * no such order: where those are applied through work vectors, each apply or
+ * solve waits for the one before it.)  An apply captured into a CUDA graph
+ * uses the same vectors: replays that hold applies of one plan must not
+ * overlap each other or other calls of that plan.
  *
  * Conventions shared with the reference (src/device/asgard_kronmult.hpp):
  *   - a Kronecker product acts on tensors of n^d entries stored contiguously,

@@ -92,3 +92,40 @@ def test_launches_of_different_sizes(cuda, kernel):
             _side_by_side([generic_job(8), generic_job(4)])
     finally:
         ab.gmres_settings(**old)
+
+
+# (d, level, terms, vectors): pair plans whose kernels held nothing between
+# calls, as lists that are applied one by one and as whole grids
+SHARED = [(2, 5, 2, "f64"), (2, 7, 4, "f64"), (5, 4, 2, "f64"), (6, 4, 1, "f64"), (3, 6, 3, "f32")]
+
+
+@pytest.mark.parametrize("d,L,T,vectors", SHARED)
+def test_one_plan_on_two_streams(cuda, d, L, T, vectors):
+    """Applies and solves of one plan that are enqueued on two streams, with
+    nothing between them, give the values of one after the other."""
+    import asgard_b200 as ab
+    import torch
+    mat = ab.SparseGridOperator(d, L, T, kind="random", seed=1).kronmult_matrix()
+    dtype = torch.float32 if vectors == "f32" else torch.float64
+    xs = [_uniform(mat.output_size(), s).to(dtype) for s in range(2)]
+    expect = [torch.empty_like(x) for x in xs]
+    for x, y in zip(xs, expect):
+        mat.apply(1.0, x, 0.0, y)
+    b = _uniform(mat.output_size(), 2)
+    dt = 1e-3 / float(expect[0].abs().max())
+    u0 = torch.zeros_like(b)
+    assert ab.simple_gmres_euler(dt, mat, u0, b, 20, 40, 1e-10, tol_mode="rel").status == 0
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = [[torch.empty_like(x) for _ in range(20)] for x in xs]
+    u = torch.zeros_like(b)
+    torch.cuda.synchronize()
+    for i in range(20):
+        for k in range(2):
+            with torch.cuda.stream(streams[k]):
+                mat.apply(1.0, xs[k], 0.0, got[k][i])
+    with torch.cuda.stream(streams[0]):
+        assert ab.simple_gmres_euler(dt, mat, u, b, 20, 40, 1e-10, tol_mode="rel").status == 0
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, expect[k]) for k in range(2) for y in got[k])
+    assert torch.equal(u, u0)
