@@ -273,13 +273,14 @@ int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
                 sweep_data **out, int64_t &bytes);
 void sweep_free(sweep_data *w);
 // Whether a pair plan of `products` pairs x terms in d dimensions is applied
-// by the tree rather than by the pair kernels.  The tree costs 2d launches
-// of 4-10 us, the pair kernels one whose time grows with the products; both
-// measured with FP64 on either side of the line: d=2 level 7, 155 and 464
-// thousand products: tree 18 and 24 us, pairs 15 and 28; d=3, 188 and 1058:
-// 32 and 37, 22 and 64; d=4, 107 and 276: 43 and 47, 31 and 60; d=5, 55 and
-// 101: 66 and 62, 56 and 94; d=6, 57 and 247: 129 and 157, 119 and 475.  The
-// pair kernels gain more from FP32.
+// by the tree rather than by the pair kernels.  The tree costs d to 2d
+// launches of 4-10 us, the pair kernels one whose time grows with the
+// products; both measured with FP64 on either side of the line: d=2 level 7,
+// 155 and 464 thousand products: tree 15 and 21 us, pairs 12 and 20, at 619
+// thousand 22 and 32; d=3, 706: 21 and 47; d=4, 107 and 276: 43 and 28, 27 and
+// 55; d=5, 55 and 101: 66 and 45, 42 and 91; d=6, 57 and 247: 129 and 154,
+// 92 and 474.  The pair kernels gain more from FP32 (d=2, 619 thousand: 20
+// and 20; d=5, 101: 37 and 55).
 inline bool sweep_pays(int d, int64_t products, bool fp32)
 {
   int64_t const least = d <= 3 ? 400000 : (d == 4 ? 262144 : 65536);

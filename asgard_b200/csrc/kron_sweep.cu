@@ -20,7 +20,9 @@
 // Y_{m + s} += L_s Y_m, which leaves the term's product in the last Y.  That
 // is 2^(m+1) - 2 half operators for a term of m dimensions, where the
 // 2^(m-1) separate chains take (m + 1) 2^(m-1) half operators: 30 against 40
-// at m = 4, 126 against 224 at m = 6.
+// at m = 4, 126 against 224 at m = 6.  The chains take fewer launches, though
+// (m, all chains and terms side by side, against 2m - 1), which decides on
+// grids of few values.
 #include "internal.cuh"
 
 #include <algorithm>
@@ -67,6 +69,7 @@ struct sweep_data
   cudaEvent_t done = nullptr;
   bool used        = false;
   int nresults = 0;
+  bool chains  = false; // lower passes write their output whole, else add to it
   sweep_units su[6][3];
   std::vector<sweep_launch> launches;
 };
@@ -86,6 +89,16 @@ constexpr int kSmall = 8;
 constexpr int kRowEntries = 16, kBlockEntries = 128;
 constexpr int kRowEntriesFew = 8, kBlockEntriesFew = 1;
 constexpr int64_t kFewValues = 1 << 18;
+// Where the terms run as separate chains: on a grid of few values, when the
+// values of the passes that the tree would share and the products to add up
+// stay few.  One FP64 apply of terms acting in every dimension, tree and
+// chains: d=3 level 6, 2 terms 33.9 and 20.8 us; d=4 level 3, 1 term 38 and
+// 25; d=5 level 4, 1 term (2.7 million extra values) 62 and 47, 3 terms (8.0
+// million) 88 and 95; d=4 level 6, 2 terms (2.5 million) 79 and 76, 4 terms
+// 122 and 130; d=6 level 1, 1 term (32 chains) 32 and 25, 3 terms (96) 34 and
+// 36, 6 terms 39 and 59.
+constexpr int64_t kChainExtra = int64_t(4) << 20;
+constexpr int kChainSums      = 64;
 
 template<typename TC> struct padW;
 template<> struct padW<double> { static constexpr int value = 10; };
@@ -345,7 +358,7 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
     k_sweep(const int4 *__restrict__ units, unit_tables tab,
             const int *__restrict__ index, const int4 *__restrict__ recs,
             const int4 *__restrict__ jobs, const TC *__restrict__ P, int T,
-            const TX *__restrict__ x, TC *__restrict__ work, int64_t N,
+            const TX *__restrict__ x, TC *__restrict__ work, int64_t N, bool lower_adds,
             const double *__restrict__ gate)
 {
   if (gate_closed(gate))
@@ -374,7 +387,7 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
   int const pstep  = D * T * padW<TC>::value;
   TC *out          = work + int64_t(job.y) * N;
   const TC *in     = work + int64_t(job.x < 0 ? 0 : job.x) * N;
-  bool const add   = fill == kSweepLower;
+  bool const add   = lower_adds && fill == kSweepLower;
   auto go          = [&](auto *src) {
     const int *cells = index + ua.z, *list = index + ub.x;
     if (ub.z > 0)
@@ -462,7 +475,7 @@ int launch_d(sweep_data const &w, const TC *P, int T, double alpha, const TX *x,
     ASGK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<D, TC, TX>, static_cast<const int4 *>(w.units), tab,
                                  static_cast<const int *>(w.index),
                                  static_cast<const int4 *>(w.recs),
-                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N, g_gate));
+                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N, !w.chains, g_gate));
     count_launch();
   }
   cfg.gridDim = dim3(int(std::min<int64_t>((w.N + 255) / 256, 148 * 8)));
@@ -554,11 +567,11 @@ std::vector<pencil_class> find_pencils(int d, int cells, const int *oned, const 
   return out;
 }
 
-// The units of one dimension and fill (see k_sweep).  A lower pass adds to
-// its output, so rows that it does not reach are left out.
+// The units of one dimension and fill (see k_sweep).  Rows that a pass does
+// not reach are left out when it adds to its output.
 void build_units(std::vector<pencil_class> const &classes, const int *lut, int R1, int F, int fill,
-                 std::vector<int4> &units, std::vector<int> &index, std::vector<int4> &recs,
-                 bool few, sweep_units &su)
+                 bool adds, std::vector<int4> &units, std::vector<int> &index,
+                 std::vector<int4> &recs, bool few, sweep_units &su)
 {
   su.first = int(units.size() / 2);
   for (auto const &c : classes)
@@ -575,7 +588,7 @@ void build_units(std::vector<pencil_class> const &classes, const int *lut, int R
       while (R < m)
         R *= 2;
       int const at = int(index.size());
-      bool any     = fill != kSweepLower;
+      bool any     = !adds;
       for (int r = 0; r < m; r++)
         for (int q = 0; q < R; q++)
         {
@@ -611,7 +624,7 @@ void build_units(std::vector<pencil_class> const &classes, const int *lut, int R
         }
       while (w.warps < kWarps && w.n > w.warps * (few ? kRowEntriesFew : kRowEntries))
         w.warps *= 2;
-      if (w.n > 0 || fill != kSweepLower)
+      if (w.n > 0 || !adds)
         rows.push_back(w);
     }
     std::stable_sort(rows.begin(), rows.end(), [](row const &a, row const &b) {
@@ -763,6 +776,66 @@ struct tree_plan
       drop(v);
     return out;
   }
+  // Every term's chains: for each subset of the dimensions above a_0 their
+  // upper parts from the last dimension down, the whole operator of a_0, the
+  // lower parts of the other dimensions upwards.  A launch takes the next pass
+  // of all of them; chains that begin alike are one until they part.
+  std::vector<int> chains(std::vector<std::vector<int>> const &terms)
+  {
+    struct link
+    {
+      int vec; // -1: the operator's x
+      const std::vector<int> *term;
+      int q;                // the last upper part was dimension a_q's
+      std::vector<int> low; // the dimensions left to their lower parts
+      int lows;             // lower parts applied, -1 before a_0's operator
+    };
+    std::vector<link> now;
+    std::vector<int> out;
+    for (auto const &t : terms)
+      now.push_back({-1, &t, int(t.size()) - 1, {}, -1});
+    while (!now.empty())
+    {
+      std::vector<link> then;
+      std::vector<int4> js;
+      auto pass = [&](link const &l, int s, int fill, link child) {
+        child.vec = take();
+        js.push_back(make_int4(l.vec, child.vec, 3 * (*l.term)[1 + s] + fill, (*l.term)[0]));
+        then.push_back(std::move(child));
+      };
+      std::vector<int> read;
+      for (auto const &l : now)
+      {
+        if (l.lows == int(l.low.size()))
+        {
+          out.push_back(l.vec);
+          continue;
+        }
+        read.push_back(l.vec);
+        if (l.lows >= 0)
+        {
+          link child = l;
+          child.lows++;
+          pass(l, l.low[l.lows], kSweepLower, std::move(child));
+          continue;
+        }
+        for (int s = l.q - 1; s >= 0; s--) // a_s next, those between go lower
+        {
+          link child = l;
+          child.q    = s;
+          for (int j = l.q - 1; j > s; j--)
+            child.low.insert(child.low.begin(), j);
+          child.lows = s == 0 ? 0 : -1;
+          pass(l, s, s == 0 ? kSweepBoth : kSweepUpper, std::move(child));
+        }
+      }
+      launch(js);
+      for (int v : read)
+        drop(v);
+      now.swap(then);
+    }
+    return out;
+  }
 };
 
 template<typename T>
@@ -814,6 +887,14 @@ int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
   w->N = int64_t(cells) * ipow3w(d);
   if (w->N >= int64_t(1) << 31) // places in a vector are 32-bit
     return ASGK_ERR_UNSUPPORTED;
+  int64_t chains = 0, extra = 0; // passes of halves beyond the tree's
+  for (auto const &t : terms)
+  {
+    int const m = int(t.size()) - 1;
+    chains += int64_t(1) << (m - 1);
+    extra += (int64_t(m + 1) << (m - 1)) - ((int64_t(2) << m) - 2);
+  }
+  w->chains = w->N < kFewValues && chains <= kChainSums && extra * w->N <= kChainExtra;
   bool used[6][3] = {};
   size_t widest   = 0;
   for (auto const &t : terms)
@@ -841,8 +922,8 @@ int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
     }
     for (int f = 0; f < 3; f++)
       if (used[k][f])
-        build_units(classes, lut, R1, int(w->N / cells / 3), f, units, index, recs,
-                    w->N < kFewValues, w->su[k][f]);
+        build_units(classes, lut, R1, int(w->N / cells / 3), f, f == kSweepLower && !w->chains,
+                    units, index, recs, w->N < kFewValues, w->su[k][f]);
     if (index.size() > size_t(1) << 30)
       return ASGK_ERR_UNSUPPORTED;
   }
@@ -851,7 +932,9 @@ int sweep_build(int d, int cells, const int *oned, const int *lut, int R1,
   tp.su   = w->su;
   tp.wide = int(std::min<int64_t>(1 << 20, kSweepBytes / (w->N * int64_t(sizeof(double)))));
   std::vector<int> last;
-  for (size_t m = 1; m <= widest; m++)
+  if (w->chains)
+    last = tp.chains(terms);
+  for (size_t m = 1; m <= widest && !w->chains; m++)
   {
     std::vector<tree_plan::node> roots;
     for (auto const &t : terms)

@@ -251,3 +251,39 @@ def test_global_cell_kernel_misaligned_and_aliasing_free_input(cuda):
         g.apply(1.0, _dev(x), 0.0, yb, precision=prec)
         torch.cuda.synchronize()
         assert torch.equal(ya, yb), prec
+
+
+# (d, level, terms, chains): several-dimension terms on both sides of the line
+# up to which they run as separate chains: few values, few of them in the
+# passes that the tree shares, few products to add up
+@pytest.mark.parametrize("d,L,T,chains", [
+    (2, 1, 2, True), (2, 6, 3, True), (2, 3, 40, False), (3, 2, 2, True), (3, 6, 2, True), (4, 1, 3, True),
+    (4, 3, 3, True), (5, 1, 2, True), (5, 4, 2, True), (6, 1, 1, True), (6, 2, 2, True), (6, 1, 4, False),
+    (6, 3, 1, False)])
+def test_chains_of_small_grids(cuda, d, L, T, chains):
+    """Terms acting in every dimension, in all but one and in one, as separate
+    chains and as the tree, against the oracle.  Separate chains take a launch
+    per dimension, one for the sum and one for the terms acting in a single
+    dimension."""
+    import asgard_b200 as ab
+    import torch
+    op = ab.SparseGridOperator(d, L, T, kind="random", seed=L)
+    pntr, indx = ab.connect_1d(L)
+    eye = (np.repeat(np.arange(len(pntr) - 1), np.diff(pntr)) == indx)[:, None] * np.eye(3).ravel()[None, :]
+    vA = op.vA.reshape(len(indx), T, d, 9).copy()
+    if T > 1:
+        vA[:, 1, d // 2] = eye          # term 1 leaves one dimension alone
+    if T > 2:
+        vA[:, 2, 1:] = eye[:, None, :]  # term 2 acts in dimension 0 only
+    vA = vA.ravel()
+    g = ab.kronmult_matrix.from_global(d, 3, L, op.table, T, vA)
+    rng = np.random.default_rng(d)
+    x, y0 = rng.uniform(-1, 1, op.N), rng.uniform(-1, 1, op.N)
+    expect = oracle.kronmult(d, 3, op.row_ptr.astype(np.int32), op.col, T, op.iA(), vA, 0.7, x, -1.3, y0.copy())
+    assert rel_err(_apply(g, 0.7, x, -1.3, y0), expect) < 1e-13
+    assert rel_err(_apply(g, 0.7, x, -1.3, y0, "fp32"), expect) < 1e-5
+    xd, yd = _dev(x), torch.zeros(op.N, dtype=torch.float64, device="cuda")
+    before = ab.launch_count()
+    g.apply(1.0, xd, 0.0, yd)
+    launches = ab.launch_count() - before
+    assert launches == d + 2 if chains else launches > d + 2
