@@ -278,12 +278,12 @@ void sweep_free(sweep_data *w);
 // products; both measured with FP64 on either side of the line: d=2 level 7,
 // 155 and 464 thousand products: tree 15 and 21 us, pairs 12 and 20, at 619
 // thousand 22 and 32; d=3, 706: 21 and 47; d=4, 107 and 276: 43 and 28, 27 and
-// 55; d=5, 55 and 101: 66 and 45, 42 and 91; d=6, 57 and 247: 129 and 154,
-// 92 and 474.  The pair kernels gain more from FP32 (d=2, 619 thousand: 20
-// and 20; d=5, 101: 37 and 55).
+// 55; d=5, 55 and 101: 66 and 45, 42 and 91; d=6, 114 and 247: 208 and 153,
+// 172 and 474.  The pair kernels gain more from FP32 (d=2, 619 thousand: 20
+// and 20; d=5, 101: 37 and 55; d=6, 114: 156 and 138, 247: 120 and 450).
 inline bool sweep_pays(int d, int64_t products, bool fp32)
 {
-  int64_t const least = d <= 3 ? 400000 : (d == 4 ? 262144 : 65536);
+  int64_t const least = d <= 3 ? 400000 : (d == 4 ? 262144 : (d == 5 ? 65536 : 163840));
   return products >= (fp32 ? least * 3 / 2 : least);
 }
 int launch_sweep(plan_data const &p, sweep_data &w, int precision, double alpha, const void *x,

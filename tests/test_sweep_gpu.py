@@ -12,10 +12,10 @@ from conftest import rel_err
 pytestmark = pytest.mark.gpu
 
 # (d, level, terms): pairs x terms on both sides of each dimension's line
-# (400 thousand for d <= 3, 262144 for d = 4, 65536 above; half as much again
-# in FP32), pencils of 1 to 128 cells
+# (400 thousand for d <= 3, 262144 for d = 4, 65536 for d = 5, 163840 above;
+# half as much again in FP32), pencils of 1 to 128 cells
 CASES = [(2, 7, 2), (2, 7, 3), (2, 7, 5), (3, 6, 1), (3, 6, 2), (4, 4, 7), (4, 5, 1), (4, 5, 2),
-         (5, 3, 7), (5, 4, 1), (6, 3, 3), (6, 3, 6)]
+         (5, 3, 7), (5, 4, 1), (6, 3, 3), (6, 3, 6), (6, 4, 1)]
 
 
 def _dev(a, dtype=None):
@@ -170,3 +170,22 @@ def test_dense_form_and_capture(cuda):
     g.replay()
     torch.cuda.synchronize()
     assert np.array_equal(yd.cpu().numpy(), _apply(dense, 1.0, x2, 0.0, np.zeros(op.N)))
+
+
+@pytest.mark.parametrize("d,L,T,precision,tree", [
+    (2, 7, 2, "fp64", False), (2, 7, 3, "fp64", True), (2, 7, 3, "fp32", False), (2, 7, 4, "fp32", True),
+    (4, 4, 6, "fp64", False), (4, 5, 1, "fp64", True), (4, 5, 1, "fp32", False), (5, 3, 6, "fp64", False),
+    (5, 4, 1, "fp64", True), (5, 4, 1, "fp32", True), (6, 3, 6, "fp64", False), (6, 3, 6, "fp32", False),
+    (6, 4, 1, "fp64", True), (6, 4, 1, "fp32", True)])
+def test_lists_that_take_the_tree(cuda, d, L, T, precision, tree):
+    """The grids on either side of each line: a launch per pass with the tree,
+    the pair kernel (and the copy of x at d = 4) below it."""
+    import asgard_b200 as ab
+    import torch
+    mat = ab.kronmult_matrix.from_grid(d, 3, L, T, ab.factor_values(d, L, T, "random"))
+    x = torch.zeros(mat.output_size(), dtype=torch.float64, device="cuda")
+    y = torch.empty_like(x)
+    before = ab.launch_count()
+    mat.apply(1.0, x, 0.0, y, precision=precision)
+    launches = ab.launch_count() - before
+    assert launches > d if tree else launches <= (2 if d == 4 else 1)
