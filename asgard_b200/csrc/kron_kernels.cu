@@ -403,20 +403,29 @@ int launch3_warps(plan_data const &p, const TC *vA, double alpha, const TX *x,
 }
 
 // Warps per output cell: a cell's warps take its pairs in turn, one latency
-// per turn, so few cells (a block each and SMs to spare) take more warps.
-// Measured, 4 / 8 / 16 warps, FP64 unless stated: d=2 level 7 (576 cells, 3
-// terms) 27.7 / 23.2 / 21.1 us; d=3 level 5 (272 cells, FP32) 16.9 / 13.0 /
-// 12.7, level 6 (688 cells) 39.5 / 41.9 / 44.1; d=4 level 4 (192 cells, FP32)
-// 21.5 / 25.2 / 25.1; d=5 level 3 (96 cells) 33.3 / 27.2 / 44.2; d=6 level 3
-// (138 cells) 119 / 95 / 152, level 4 (501 cells) 1193 / 1219 / 1966.
+// per turn, so few cells (a block each and SMs to spare) with more pairs than
+// four warps take in a turn or two take more warps.  One apply replayed from a
+// graph, 4 / 16 warps, FP64, d=2: 48 cells of 42 pairs 4.3 / 5.1 us, 112 of
+// 81 pairs 5.3 / 5.2, 576 cells and 3 terms 26.5 / 20.2, 2816 cells and one
+// term 92.5 / 98.0, three terms 230 / 214.  4 / 8 warps: d=3, FP32 vectors,
+// 38 cells of 38 pairs and 3 terms 5.1 / 5.5, 104 of 97 pairs 5.8 / 5.2, 272
+// cells 15.3 / 12.0, 688 cells (FP64) 39.5 / 41.9; d=4, FP32 vectors, 19 cells
+// of 19 pairs 5.3 / 5.7, 63 of 63 8.5 / 7.0, 192 cells 21.5 / 25.2; d=5 6
+// cells of 6 pairs 4.6 / 5.0, 26 of 26 7.8 / 7.1, 96 cells 31.7 / 25.9; d=6 7
+// cells 6.4 / 5.3, 138 cells 117 / 93, 501 cells 1193 / 1219.
 template<int D, typename TC, typename TX, typename TY, index_mode MODE,
          bool EULER>
 int launch3(plan_data const &p, const TC *vA, double alpha, const TX *x,
             double beta, TY *y, double ex, cudaStream_t s)
 {
+  constexpr int kManyPairs = D <= 3 ? 64 : (D == 4 ? 32 : (D == 5 ? 8 : 0));
+  bool const many          = p.nnz >= int64_t(kManyPairs) * p.rows;
   if constexpr (D == 2)
-    return launch3_warps<D, TC, TX, TY, MODE, EULER, 16>(p, vA, alpha, x, beta, y, ex, s);
-  else if (p.rows <= (D == 3 ? 2 : 1) * 148)
+  {
+    if (many && (p.rows <= 2048 || p.terms > 1))
+      return launch3_warps<D, TC, TX, TY, MODE, EULER, 16>(p, vA, alpha, x, beta, y, ex, s);
+  }
+  else if (many && p.rows <= (D == 3 ? 2 : 1) * 148)
     return launch3_warps<D, TC, TX, TY, MODE, EULER, 8>(p, vA, alpha, x, beta, y, ex, s);
   return launch3_warps<D, TC, TX, TY, MODE, EULER, 4>(p, vA, alpha, x, beta, y, ex, s);
 }

@@ -496,15 +496,17 @@ int launch_staged_warps(plan_data const &p, const TC *vF, double alpha,
   return ASGK_OK;
 }
 
-// four warps per output cell, eight where the cells leave SMs idle (d=4
-// level 3, 63 cells, 6 terms: 23.0 -> 18.9 us; d=3 level 4, 104 cells: 16.8
-// -> 14.8; d=4 level 4, 192 cells, 3 terms, with eight: 31.2 -> 35.7)
+// four warps per output cell, eight where the cells leave SMs idle and, at
+// d=3, have pairs for them (d=4 level 3, 63 cells, 6 terms: 23.0 -> 18.9 us;
+// d=3 level 4, 104 cells of 97 pairs: 16.8 -> 14.8; level 3, 38 cells of 38
+// pairs, with eight: 5.8 -> 6.3 replayed from a graph; d=4 level 4, 192 cells,
+// 3 terms, with eight: 31.2 -> 35.7)
 template<int D, typename TC, index_mode MODE, bool EULER>
 int launch_staged_t(plan_data const &p, const TC *vF, double alpha,
                     const TC *xp, const double *x, double beta, double *y,
                     double ex, cudaStream_t s)
 {
-  if (p.rows <= 148)
+  if (p.rows <= 148 && (D > 3 || p.nnz >= int64_t(64) * p.rows))
     return launch_staged_warps<D, TC, MODE, EULER, 2 * kStagedWarps>(p, vF, alpha, xp, x, beta, y,
                                                                      ex, s);
   return launch_staged_warps<D, TC, MODE, EULER, kStagedWarps>(p, vF, alpha, xp, x, beta, y, ex, s);

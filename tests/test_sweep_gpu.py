@@ -189,3 +189,25 @@ def test_lists_that_take_the_tree(cuda, d, L, T, precision, tree):
     mat.apply(1.0, x, 0.0, y, precision=precision)
     launches = ab.launch_count() - before
     assert launches > d if tree else launches <= (2 if d == 4 else 1)
+
+
+@pytest.mark.parametrize("d,L,T", [(2, 2, 1), (2, 4, 3), (2, 5, 1), (2, 9, 1), (2, 9, 2), (3, 3, 1), (3, 4, 1),
+                                   (3, 5, 2), (4, 3, 2), (5, 3, 1), (5, 4, 1), (6, 3, 1), (6, 4, 1)])
+def test_pair_kernels_beside_a_whole_grid(cuda, d, L, T):
+    """Lists with one pair dropped, from a few cells to several thousand: the
+    pair kernels with every number of warps per cell, FP64, FP32 and FP32
+    vectors, against the oracle."""
+    import asgard_b200 as ab
+    import torch
+    op = ab.SparseGridOperator(d, L, T, kind="random", seed=1)
+    at = int(op.row_ptr[1]) - 1
+    ptr = op.row_ptr.copy()
+    ptr[1:] -= 1
+    col, conn = np.delete(op.col, at), np.delete(op.conn, at, axis=0)
+    mat = ab.kronmult_matrix.from_conn(d, 3, op.rows, op.rows, T, ptr, col, conn, op.vA)
+    rng = np.random.default_rng(L)
+    x, y0 = rng.uniform(-1, 1, op.N), rng.uniform(-1, 1, op.N)
+    expect = _expect(op, ptr, col, conn, 0.7, x, -1.3, y0)
+    assert rel_err(_apply(mat, 0.7, x, -1.3, y0), expect) < 1e-13
+    assert rel_err(_apply(mat, 0.7, x, -1.3, y0, "fp32"), expect) < 1e-5
+    assert rel_err(_apply(mat, 0.7, x, -1.3, y0, "fp32", torch.float32), expect) < 1e-5
