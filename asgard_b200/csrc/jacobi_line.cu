@@ -377,15 +377,29 @@ constexpr int kSplit      = 4;
 constexpr int kSplitItems = 32; // (4-row block, group) items of a CTA, a lane each
 constexpr int kSplitTile  = 64; // matrix rows per staged tile
 // The pencils that clusters take, multiples of 4 kSplit cells: all that the
-// small-pencil kernel leaves while the clusters are resident at once (no
-// third launch), else the long ones, else none.  Level 7 solves without
-// with clusters: d=2 1.55 and 1.15 ms, d=3 1.67 and 1.27, d=4 6.16 and 3.76;
-// d=5 level 6 4.23 and 3.73.  On large vectors the rest of a factor covers
-// the chain and the copies only cost: d=6 level 6 7.3 and 7.9 ms, level 7
-// 21.1 and 21.8.
+// small-pencil kernel leaves while there are few clusters (no third launch),
+// else the long ones, else none.  Level 7 solves without and with clusters:
+// d=2 1.55 and 1.15 ms, d=3 1.67 and 1.27, d=4 6.16 and 3.56; d=5 level 6
+// 4.27 and 3.69.  On large vectors the rest of a factor covers the chain and
+// the copies only cost: d=6 level 6 7.3 and 7.9 ms, level 7 21.1 and 21.8.
+// (kSplitUnits clusters are two CTAs per SM; in FP64 with several line
+// dimensions one CTA fits an SM, and more than 37 clusters queue.)
 constexpr int kSplitMinM       = 64;
 constexpr int kSplitUnits      = 2 * 148 / kSplit;
 constexpr int64_t kSplitValues = 1 << 20;
+// A launch uses them while the longest pencil's chain (its matrix: cells^2)
+// is what the factor waits for, up to so many values of the vector per
+// cells^2; beyond, in recorded cycles, the clusters cost more than they save,
+// and their units run as one CTA each.  Solves without and with clusters:
+// FP64, M line dimensions, values / longest^2 = 61 (d=4 level 4, M=2) 1.31 and
+// 1.20 ms; 30 (d=4 level 6) M=1 1.03 and 0.82; 176 (d=5 level 6) M=2 5.03 and
+// 4.15, M=1 1.55 and 1.56 (an apply 38 and 44 us); 238 (d=5 level 5) M=2 2.36
+// and 2.48, M=1 0.72 and 0.76; 305 (d=5 level 4) 1.44 and 1.61; 1427 (d=6
+// level 4, M=3) 3.21 and 3.74.  FP32: 176 M=1 1.88 and 1.80; 238 M=1 1.06 and
+// 1.08, M=2 2.28 and 2.12; 305 M=1 0.78 and 0.79, M=2 1.53 and 1.46; 1427 2.64
+// and 2.86.
+template<typename R, int M>
+constexpr int64_t kSplitShare = (sizeof(R) == 4 ? 200 : 100) * (M > 1 ? 2 : 1);
 inline bool line_splits(int m)
 {
   return m % (4 * kSplit) == 0 && 3 * m / (4 * kSplit) <= kSplitItems;
@@ -1186,6 +1200,7 @@ struct line_factor
   int nsplit = 0;   // the first of them, a cluster each
   int split_rows = 0, split_tile = 0; // their largest Rp * G; rows per CTA
   int split_sums = 0;                 // and rows per CTA * groups
+  int split_rp = 0, longest = 0;      // their largest Rp; cells of the longest
   int max_rows = 0; // largest Rp * G of its units (shared memory)
   int max_rp   = 0; // largest padded pencil size (matrix tiles)
   int nbatches = 0; // batches of pencils of 1, 2, 4 or 8 cells
@@ -1474,7 +1489,7 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
     int max_rp       = 0;
     std::vector<int4> units, batches, bcells;
     int max_rows = 0;
-    int nsplit = 0, split_rows = 0, split_tile = 0, split_sums = 0;
+    int nsplit = 0, split_rows = 0, split_tile = 0, split_sums = 0, split_rp = 0, longest = 0;
     for (size_t pe = 0; pe < pen_m.size();)
     {
       int const m = pen_m[pe];
@@ -1515,6 +1530,8 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
           split_sums = std::max(split_sums, 4 * nb * gc);
         }
         split_tile = std::max(split_tile, 4 * nb);
+        split_rp   = std::max(split_rp, Rp);
+        longest    = std::max(longest, m);
         ++pe;
         continue;
       }
@@ -1536,6 +1553,7 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes)
     fac->nbatches = int(batches.size());
     fac->nsplit   = nsplit, fac->split_rows = split_rows;
     fac->split_tile = split_tile, fac->split_sums = split_sums;
+    fac->split_rp = split_rp, fac->longest = longest;
     int rc;
     if ((rc = upload(&fac->units, units, bytes)) || (rc = upload(&fac->batches, batches, bytes)) ||
         (rc = upload(&fac->bcells, bcells, bytes)) ||
@@ -1601,13 +1619,18 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
   for (int q = 0; q < 3; q++)
     a.st_line[q] = q < M ? ipow3l(D - 1 - ld.line[q]) : 0;
   // the launches of the factor, the first on the caller's stream
-  int const nlarge = f.nunits - f.nsplit;
-  int const parts  = (f.nsplit > 0) + (nlarge > 0) + (f.nbatches > 0);
+  int64_t const values = int64_t(ld.rows) * ipow3l(D);
+  int const nsplit =
+      values <= kSplitShare<R, M> * f.longest * f.longest ? f.nsplit : 0;
+  int const nlarge   = f.nunits - nsplit;
+  int const max_rows = nsplit > 0 ? f.max_rows : std::max(f.max_rows, f.split_rows);
+  int const max_rp   = nsplit > 0 ? f.max_rp : std::max(f.max_rp, f.split_rp);
+  int const parts    = (nsplit > 0) + (nlarge > 0) + (f.nbatches > 0);
   if (parts > 1)
     ASGK_CUDA(cudaEventRecord(ld.fork[KIDX], s));
   cudaStream_t const s_split = s;
-  cudaStream_t const s_large = f.nsplit > 0 ? ld.side : s;
-  cudaStream_t const s_small = f.nsplit > 0 && nlarge > 0 ? ld.side2
+  cudaStream_t const s_large = nsplit > 0 ? ld.side : s;
+  cudaStream_t const s_small = nsplit > 0 && nlarge > 0 ? ld.side2
                                : (parts > 1 ? ld.side : s);
   auto fork = [&](cudaStream_t to) -> int {
     if (to != s)
@@ -1628,7 +1651,7 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
     return ((12 * (size_t(rows) / 3 + 1) + 15) / 16) * 16 +
            sizeof(R) * (2 * size_t(rows) * NCP + tiles);
   };
-  if (f.nsplit > 0)
+  if (nsplit > 0)
   {
     size_t const shm =
         shared(f.split_rows, std::max(2 * size_t(kSplitTile) * f.split_tile,
@@ -1641,7 +1664,7 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
     cl.val.clusterDim.x = kSplit;
     cl.val.clusterDim.y = cl.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim          = dim3(kSplit * f.nsplit);
+    cfg.gridDim          = dim3(kSplit * nsplit);
     cfg.blockDim         = dim3(kLineThreads);
     cfg.dynamicSmemBytes = shm;
     cfg.stream           = s_split;
@@ -1655,12 +1678,12 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
   {
     if (int rc = fork(s_large))
       return rc;
-    size_t const shm = shared(f.max_rows, 2 * size_t(kLineTile) * f.max_rp);
+    size_t const shm = shared(max_rows, 2 * size_t(kLineTile) * max_rp);
     auto kern        = k_line_factor<R, D, M, KIDX, 1>;
     static int const most = shared_ceiling(reinterpret_cast<const void *>(kern));
     ASGK_CUDA(allow_shared(kern, most));
     line_args<R> al = a;
-    al.units += f.nsplit;
+    al.units += nsplit;
     kern<<<nlarge, kLineThreads, shm, s_large>>>(al, in64, inR, out64, outR, bj ? 1 : 0,
                                                  sc, vscale, vc, zc, g_gate);
     ASGK_LAUNCHED();

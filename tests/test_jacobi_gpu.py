@@ -316,7 +316,7 @@ def _line_by_eigh(op, dt, v):
 
 
 @pytest.mark.parametrize("d,L,T", [(2, 4, 2), (2, 6, 2), (2, 7, 2), (3, 7, 3), (4, 5, 4), (4, 6, 4), (4, 7, 4),
-                                   (5, 6, 5), (6, 5, 6), (6, 6, 6)])
+                                   (5, 6, 5), (6, 5, 6), (6, 6, 6), (5, 4, 2), (5, 4, 5), (5, 5, 5), (6, 4, 6)])
 def test_line_jacobi_long_pencils(cuda, d, L, T):
     """Pencils of 16 to 128 cells, those that a cluster of CTAs shares and
     those that one CTA takes (1 to 3 line dimensions), against NumPy in FP64.
