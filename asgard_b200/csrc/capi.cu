@@ -362,7 +362,9 @@ int attach_sweep(plan_data &p, grid_cells const &g)
       terms[t].push_back(k);
   }
   int rc = ASGK_OK;
-  if (p.vP64 == nullptr) // the expanded form
+  bool const expanded = p.vP64 == nullptr; // no factors by connection yet
+  int64_t const held  = p.device_bytes;
+  if (expanded)
   {
     int64_t const blk = int64_t(p.d) * p.terms * 9;
     if ((rc = dev_alloc(&p.vP64, p.vA_len / blk * p.d * p.terms * 10, p.device_bytes)) == ASGK_OK)
@@ -373,6 +375,15 @@ int attach_sweep(plan_data &p, grid_cells const &g)
   if (rc == ASGK_OK)
     rc = sweep_build(p.d, p.rows, g.oned.data(), g.lut.data(), g.R, terms, true, &p.sweep,
                      p.device_bytes);
+  if (rc != ASGK_OK && expanded)
+  {
+    cudaFree(p.vP64);
+    cudaFree(p.vP32);
+    p.vP64         = nullptr;
+    p.vP32         = nullptr;
+    p.nconn        = 0;
+    p.device_bytes = held;
+  }
   return (rc == ASGK_ERR_UNSUPPORTED || rc == ASGK_ERR_ALLOC) ? int(ASGK_OK) : rc;
 }
 

@@ -211,3 +211,33 @@ def test_pair_kernels_beside_a_whole_grid(cuda, d, L, T):
     assert rel_err(_apply(mat, 0.7, x, -1.3, y0), expect) < 1e-13
     assert rel_err(_apply(mat, 0.7, x, -1.3, y0, "fp32"), expect) < 1e-5
     assert rel_err(_apply(mat, 0.7, x, -1.3, y0, "fp32", torch.float32), expect) < 1e-5
+
+
+def test_expanded_list_without_a_tree_holds_no_factor_copies(cuda):
+    """The whole connectivity of a grid that is not closed below runs on the
+    pair kernels; as an expanded list it holds what a list with a pair missing
+    holds, but for that pair."""
+    import asgard_b200 as ab
+    d, L, T = 4, 6, 1
+    op = ab.SparseGridOperator(d, L, T, kind="random", seed=1)
+    keep = ~((op.table[:, 0] == 0) & (op.table[:, 1:d].sum(axis=1) > 1))
+    new = np.cumsum(keep) - 1
+    rows = np.repeat(np.arange(op.rows), np.diff(op.row_ptr))
+    on = keep[rows] & keep[op.col]
+    cells = int(keep.sum())
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(new[rows[on]], minlength=cells))]).astype(np.int64)
+    col, conn = new[op.col[on]].astype(np.int32), op.conn[on]
+    assert len(col) * T >= 262144       # enough pairs for the tree
+
+    def plan(ptr, col, conn):
+        return ab.kronmult_matrix.from_csr(d, 3, cells, cells, T, ptr, col, ab.expand_iA(conn, d, 3, T), op.vA)
+    less = ptr.copy()
+    less[1:] -= 1
+    at = int(ptr[1]) - 1
+    mat = plan(ptr, col, conn)
+    missing = plan(less, np.delete(col, at), np.delete(conn, at, axis=0))
+    assert mat.device_bytes() == missing.device_bytes() + 4 * (1 + T * d)
+    rng = np.random.default_rng(2)
+    x, y0 = rng.uniform(-1, 1, cells * 81), rng.uniform(-1, 1, cells * 81)
+    expect = _expect(op, ptr, col, conn, -0.5, x, 2.0, y0)
+    assert rel_err(_apply(mat, -0.5, x, 2.0, y0), expect) < 1e-13
