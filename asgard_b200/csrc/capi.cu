@@ -316,11 +316,18 @@ bool find_grid(int d, int rows, std::vector<int64_t> const &row_ptr, const int *
   bool ok = true;
 #pragma omp parallel
   {
-    std::vector<int> seen(rows, -1);
+    std::vector<int> seen;
+    try // nothing may leave a thread of the team
+    {
+      seen.assign(rows, -1);
+    }
+    catch (std::bad_alloc const &)
+    {
+    }
 #pragma omp for schedule(dynamic, 16)
     for (int r = 0; r < rows; r++)
     {
-      bool good     = true;
+      bool good     = !seen.empty();
       const int *er = &g.oned[size_t(r) * d];
       for (int64_t p = row_ptr[r]; p < row_ptr[r + 1] && good; p++)
       {
