@@ -346,3 +346,26 @@ def test_device_built_pairs_match_host_built(cuda, d, L, T):
     md.apply_euler(1e-3, -1.0, x, 0.5, yb)
     torch.cuda.synchronize()
     assert np.array_equal(ya.cpu().numpy(), yb.cpu().numpy())
+
+
+@pytest.mark.parametrize("d,L", [(4, 7), (6, 5)])
+def test_device_built_pairs_of_large_grids(cuda, d, L):
+    """The pair list that asgk_plan_create_grid writes for a grid large enough
+    for n = 3 plans not to read it in an apply: with n = 2 every pair is read
+    in the list's order, so equal bits are equal lists."""
+    import asgard_b200 as ab
+    import torch
+    table = ab.sparse_grid(d, L)
+    cells = table.shape[0]
+    row_ptr, col, conn = ab.build_pairs(d, L, table)
+    rng = np.random.default_rng(L)
+    vA = rng.uniform(-1, 1, len(ab.connect_1d(L)[1]) * d * 4)
+    mh = ab.kronmult_matrix.from_conn(d, 2, cells, cells, 1, row_ptr, col, conn, vA)
+    md = ab.kronmult_matrix.from_grid(d, 2, L, 1, vA)
+    assert md.num_pairs() == mh.num_pairs() == len(col)
+    x = to_dev(rng.uniform(-1, 1, cells * 2 ** d))
+    ya, yb = torch.empty_like(x), torch.empty_like(x)
+    mh.apply(1.0, x, 0.0, ya)
+    md.apply(1.0, x, 0.0, yb)
+    assert torch.isfinite(ya).all() and ya.abs().max() > 0
+    assert torch.equal(ya, yb)
