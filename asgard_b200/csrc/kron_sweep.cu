@@ -69,7 +69,7 @@ struct sweep_data
   cudaEvent_t done = nullptr;
   bool used        = false;
   int nresults = 0;
-  bool chains  = false; // lower passes write their output whole, else add to it
+  bool chains  = false; // separate chains, not a tree
   sweep_units su[6][3];
   std::vector<sweep_launch> launches;
 };
@@ -341,10 +341,10 @@ large_pencil(const int4 *__restrict__ recs, int rounds, const int *__restrict__ 
 }
 
 // One launch of the tree: blockIdx.y is a job (input vector, -1 the operator's
-// x; output vector; 3 * dimension + fill; term), blockIdx.x a range of the
-// units of its dimension and fill.  Pencils that hold the same 1D cells form
-// a class and share every index and factor below the cells themselves; a
-// class's columns are its pencils' fibres (3^(d-1) each), 32 to a tile, one
+// x; 2 * output vector, odd to add to it; 3 * dimension + fill; term),
+// blockIdx.x a range of the units of its dimension and fill.  Pencils that
+// hold the same 1D cells form a class and share every index and factor below
+// the cells themselves; a class's columns are its pencils' fibres (3^(d-1) each), 32 to a tile, one
 // to a lane, so a warp's factors are uniform and no lane is idle whatever d.
 // Pencils of up to kSmall cells: kSmall cell fibres per lane, the shorter the
 // pencils the more tiles.  Bound by the vectors' traffic through L2 (DRAM
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
     k_sweep(const int4 *__restrict__ units, unit_tables tab,
             const int *__restrict__ index, const int4 *__restrict__ recs,
             const int4 *__restrict__ jobs, const TC *__restrict__ P, int T,
-            const TX *__restrict__ x, TC *__restrict__ work, int64_t N, bool lower_adds,
+            const TX *__restrict__ x, TC *__restrict__ work, int64_t N,
             const double *__restrict__ gate)
 {
   if (gate_closed(gate))
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
   // {entries, first record, rounds} or {connections, cells at most, 0}
   int64_t const u = 2 * (int64_t(su.first) + blockIdx.x);
   int4 const ua = __ldg(units + u), ub = __ldg(units + u + 1);
-  int const k = job.z / 3, fill = job.z - 3 * k;
+  int const k = job.z / 3;
   int stride  = 1;
 #pragma unroll
   for (int j = 1; j < D; j++)
@@ -385,9 +385,9 @@ __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
       stride *= 3;
   const TC *Pk     = P + (int64_t(k) * T + job.w) * padW<TC>::value;
   int const pstep  = D * T * padW<TC>::value;
-  TC *out          = work + int64_t(job.y) * N;
+  TC *out          = work + int64_t(job.y >> 1) * N;
   const TC *in     = work + int64_t(job.x < 0 ? 0 : job.x) * N;
-  bool const add   = lower_adds && fill == kSweepLower;
+  bool const add   = (job.y & 1) != 0;
   auto go          = [&](auto *src) {
     const int *cells = index + ua.z, *list = index + ub.x;
     if (ub.z > 0)
@@ -475,7 +475,7 @@ int launch_d(sweep_data const &w, const TC *P, int T, double alpha, const TX *x,
     ASGK_CUDA(cudaLaunchKernelEx(&cfg, k_sweep<D, TC, TX>, static_cast<const int4 *>(w.units), tab,
                                  static_cast<const int *>(w.index),
                                  static_cast<const int4 *>(w.recs),
-                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N, !w.chains, g_gate));
+                                 static_cast<const int4 *>(w.jobs + l.job0), P, T, x, work, w.N, g_gate));
     count_launch();
   }
   cfg.gridDim = dim3(int(std::min<int64_t>((w.N + 255) / 256, 148 * 8)));
@@ -730,7 +730,7 @@ struct tree_plan
       for (auto const &q : in)
       {
         out.push_back(take());
-        js.push_back(make_int4(q.vec, out.back(), 3 * (*q.term)[1] + kSweepBoth, (*q.term)[0]));
+        js.push_back(make_int4(q.vec, 2 * out.back(), 3 * (*q.term)[1] + kSweepBoth, (*q.term)[0]));
       }
       launch(js);
       return out;
@@ -746,7 +746,7 @@ struct tree_plan
     for (auto const &q : in)
     {
       up.push_back({take(), q.term});
-      js.push_back(make_int4(q.vec, up.back().vec, 3 * (*q.term)[1 + s] + kSweepUpper, (*q.term)[0]));
+      js.push_back(make_int4(q.vec, 2 * up.back().vec, 3 * (*q.term)[1 + s] + kSweepUpper, (*q.term)[0]));
     }
     launch(js);
     std::vector<int> low;
@@ -769,7 +769,7 @@ struct tree_plan
     }
     js.clear();
     for (size_t i = 0; i < in.size(); i++)
-      js.push_back(make_int4(low[i], out[i], 3 * (*in[i].term)[1 + s] + kSweepLower,
+      js.push_back(make_int4(low[i], 2 * out[i] + 1, 3 * (*in[i].term)[1 + s] + kSweepLower,
                              (*in[i].term)[0]));
     launch(js);
     for (int v : low)
@@ -800,7 +800,7 @@ struct tree_plan
       std::vector<int4> js;
       auto pass = [&](link const &l, int s, int fill, link child) {
         child.vec = take();
-        js.push_back(make_int4(l.vec, child.vec, 3 * (*l.term)[1 + s] + fill, (*l.term)[0]));
+        js.push_back(make_int4(l.vec, 2 * child.vec, 3 * (*l.term)[1 + s] + fill, (*l.term)[0]));
         then.push_back(std::move(child));
       };
       std::vector<int> read;
