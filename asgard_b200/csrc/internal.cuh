@@ -263,7 +263,8 @@ int launch_global(plan_data const &p, int precision, double alpha,
                   cudaStream_t s);
 
 // kron_sweep.cu: terms acting in several dimensions as a tree of 1D passes.
-// Vectors the tree may hold at once (beyond what one path needs): fewer make
+// Bytes of vectors the tree may hold at once (beyond what one path needs), per
+// plan and from its creation: fewer make
 // its launches too small, more gain nothing.  64 / 256 / 768 / 1536 MB: d=4
 // level 7, 4 terms 402 / 254 / 254 / 254 us; d=6 level 5, 6 terms 4888 / 3702 /
 // 2953 / 2953 us.

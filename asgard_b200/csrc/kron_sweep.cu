@@ -347,12 +347,14 @@ large_pencil(const int4 *__restrict__ recs, int rounds, const int *__restrict__ 
 // the cells themselves; a class's columns are its pencils' fibres (3^(d-1) each), 32 to a tile, one
 // to a lane, so a warp's factors are uniform and no lane is idle whatever d.
 // Pencils of up to kSmall cells: kSmall cell fibres per lane, the shorter the
-// pencils the more tiles.  Bound by the vectors' traffic through L2 (DRAM
-// where they exceed it) on large grids, by a launch's chain of loads on small
-// ones.  One FP64 apply, all launches: d=4 level 7, 4 terms 254 us (5305 by
-// the pair kernel); d=6 level 5, 6 terms 2.95 ms (21.8); d=3 level 6, 2 terms
-// 39 us (129 as separate chains, a thread per output entry).  Two blocks per
-// SM: more spill the fibres (d=4 277 -> 320-500 us with three or four).
+// pencils the more tiles.  Bound by the latency of its loads at two blocks of
+// 126 registers per SM, 23 % of the warps: the widest launches use the
+// load/store pipe to 59 % (d=4 level 7) and 47 % (d=6 level 5, where DRAM moves
+// 3.4 TB/s), narrow ones wait for one chain of loads.  One FP64 apply, all
+// launches: d=4 level 7, 4 terms 254 us (5305 by the pair kernel); d=6 level
+// 5, 6 terms 2.96 ms (21.8); d=3 level 6, 2 terms, as separate chains 28 us
+// (129 with a kernel of a thread per output entry).  Two blocks per SM: more
+// spill the fibres (d=4 277 -> 320-500 us with three or four).
 template<int D, typename TC, typename TX>
 __global__ void __launch_bounds__(kWarps * 32, kSweepBlocks)
     k_sweep(const int4 *__restrict__ units, unit_tables tab,

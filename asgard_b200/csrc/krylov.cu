@@ -772,13 +772,16 @@ __global__ void k_store_basis(double *__restrict__ w, float *__restrict__ vf,
 // ---- a whole Gram-Schmidt step of a short basis in one launch -----------
 //
 // For vectors of up to kStepRows values the two passes above are a few
-// microseconds of launch and reduction latency each.  One cluster of kStepCtas CTAs does the step: every CTA
-// holds its rows of w in shared memory, sends its partial projections (a
-// warp per column) and its part of ||w||^2 to the others' shared memory, and
-// adds them in rank order, so the sums have a fixed order.  h[0..k) and
-// h[k] = ||w||^2 as the passes leave them; ga as in k_update_norm_h.  Four
-// plain GMRES time steps on 2304 values: 15.5 -> 14.6 ms; two on 7344 took
-// 8.07 ms with the passes and 8.51 in one launch, so the line lies between.
+// microseconds of launch and reduction latency each.  One cluster of
+// kStepCtas CTAs does the step: every CTA holds its rows of w in shared
+// memory, sends its partial projections (a warp per column) and its part of
+// ||w||^2 to the others' shared memory, and adds them in rank order, so the
+// sums have a fixed order.  h[0..k) and h[k] = ||w||^2 as the passes leave
+// them; ga as in k_update_norm_h.  Four plain GMRES time steps on 2304 values:
+// 15.5 -> 14.6 ms; two on 7344 took 8.07 ms with the passes and 8.51 in one
+// launch, so the line lies between.  The same solve at the line, 4095 values
+// in one launch and 4104 by the passes: FP64 26.0 and 28.7 ms, with an FP32
+// basis 12.8 and 15.0.
 constexpr int kStepCtas      = 8;
 constexpr int kStepThreads   = 512;
 constexpr int64_t kStepRows  = 4096;

@@ -7,9 +7,13 @@
 Builds the operator (advection/diffusion factors unless --kind random), runs
 --warmup untimed applies of the fused backward-Euler operator
 y = x - dt*K*x, then --reps timed applies (CUDA events on the launching
-stream) and prints one JSON line: ms per launch, algorithmic TFLOP/s
-(2*d*T*n^(d+1) flops per pair -- every cell pair in the dense form;
-2*n^(d+1) per single-direction pair in the global form) and the fraction of the measured FMA peak.
+stream) and prints one JSON line: ms and launches per apply, algorithmic GB/s
+(x read once, y written) and, where an apply is one pass over its pairs,
+TFLOP/s (2*d*T*n^(d+1) flops per pair -- every cell pair in the dense form;
+2*n^(d+1) per single-direction pair in the global form) and the fraction of
+the measured FMA peak.  Terms acting in several dimensions and the pair lists
+of whole grids run as a tree of 1D passes (an apply of more than two
+launches), which does not perform the pairs' flops: they stand as pair_flops.
 The kernel summaries of this repository were taken with this command under ncu.
 """
 from __future__ import annotations
@@ -28,7 +32,7 @@ def main():
     ap.add_argument("--kind", default="advdiff")
     ap.add_argument("--precision", default="fp64", choices=["fp64", "fp32", "bf16"])
     ap.add_argument("--reps", type=int, default=3)
-    ap.add_argument("--warmup", type=int, default=1)
+    ap.add_argument("--warmup", type=int, default=1, help="untimed applies (at least one)")
     ap.add_argument("--peak", action="store_true", help="also measure the FMA peak")
     ap.add_argument("--device-build", action="store_true",
                     help="connected pairs found on the GPU (from_grid) instead of "
@@ -82,7 +86,10 @@ def main():
                           "algorithmic_GBps": 16 * op.N / ms / 1e6,
                           "device_bytes": pc.device_bytes()}))
         return
-    for _ in range(args.warmup):
+    before = ab.launch_count()
+    mat.apply_euler(1e-3, 1.0, x, 0.0, y, precision=args.precision)
+    launches = ab.launch_count() - before
+    for _ in range(args.warmup - 1):
         mat.apply_euler(1e-3, 1.0, x, 0.0, y, precision=args.precision)
     torch.cuda.synchronize()
     e0 = torch.cuda.Event(enable_timing=True)
@@ -97,9 +104,16 @@ def main():
     out = {"d": args.d, "level": args.level, "terms": args.terms, "mode": args.mode,
            "num_pairs": mat.num_pairs(),
            "precision": args.precision, "cells": op.rows, "pairs": op.nnz,
-           "dofs": op.N, "ms_per_launch": ms, "tflops": flops / ms / 1e9,
-           "flops_per_launch": flops, "setup_s": t_setup,
+           "dofs": op.N, "ms_per_apply": ms, "launches_per_apply": launches,
+           "algorithmic_GBps": 16 * op.N / ms / 1e6, "setup_s": t_setup,
            "device_bytes": mat.device_bytes()}
+    # the tensor-core form takes a launch per class of pencils
+    tree = launches > 2 and args.precision != "bf16"
+    if tree:
+        out["pair_flops"] = flops
+    else:
+        out["flops_per_apply"] = flops
+        out["tflops"] = flops / ms / 1e9
     if args.precision != "fp64":
         # the low-precision product K x against the FP64 one on the same x
         y64, ylo = torch.zeros_like(x), torch.zeros_like(x)
@@ -107,7 +121,7 @@ def main():
         mat.apply(1.0, x, 0.0, ylo, precision=args.precision)
         torch.cuda.synchronize()
         out["rel_err_vs_fp64"] = float(torch.linalg.norm(ylo - y64) / torch.linalg.norm(y64))
-    if args.peak:
+    if args.peak and not tree:
         pk = C.c_double()
         ab.lib.asgk_measure_fma_peak(0 if args.precision == "fp64" else 1, C.byref(pk))
         out["fma_peak_tflops"] = pk.value

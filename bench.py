@@ -18,12 +18,11 @@ refinement.  Timed beside it: the plain
 baseline -- FP64 GMRES with the connected-pair FP64 kronmult (one solve by
 default) -- and, at d <= 4, the same method on the
 connected-pair operator.  Inputs are resident in HBM when the timed region
-starts; at d=6 every vector (94 MB) and the plain baseline's pair list
-(6.3 GB) are larger than L2, at d=4 the method's working set is L2-sized by
-design; no extra L2 flush is done between steps.  ``e2e`` is the same
-solves with b in pinned host memory and x read back into pinned host
-memory every step, the copies on a second stream overlapping the
-neighbouring steps' solves.
+starts; at d=6 a solve's vectors (94 MB each, over 2 GB with the Krylov
+basis) are larger than L2, at d=4 the working set is L2-sized by design; no
+extra L2 flush is done between steps.  ``e2e`` is the same solves with b in
+pinned host memory and x read back into pinned host memory every step, the
+copies on a second stream overlapping the neighbouring steps' solves.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
@@ -60,11 +59,11 @@ RESTART = 50
 TOL = 1e-10
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of
-# each workload's operator kernels, from one ncu capture of that kernel on
+# each workload's method operator, from one ncu capture of that kernel on
 # that workload; None where no capture was taken.
 KERNEL_TRAFFIC = {
-    ("global", "d4"): 3_930_368,
-    ("global", "d6"): 71_265_792 + 54_134_016,
+    "d4": 3_930_368,
+    "d6": 71_265_792 + 54_134_016,
 }
 
 
@@ -220,10 +219,9 @@ def _config(workload):
                         f"restart {RESTART}, rel tol {TOL}",
             "d": cfg["d"], "n": 3, "level": cfg["level"], "terms": cfg["terms"],
             "dt": cfg["dt"], "nu": cfg["nu"], "restart": RESTART, "tol": TOL,
-            "l2": ("vectors (94 MB) and the plain baseline's pair list larger "
-                   "than L2; no flush" if cfg["d"] >= 6 else
-                   "plain baseline's pair list larger than L2; the method's "
-                   "working set L2-sized; no flush")}
+            "l2": ("a solve's vectors (94 MB each, over 2 GB with the Krylov "
+                   "basis) larger than L2; no flush"
+                   if cfg["d"] >= 6 else "working set L2-sized; no flush")}
 
 
 # ---------------------------------------------------------------- reference arm
@@ -721,11 +719,9 @@ def rooflines(ab, op, mat, gmat, method, dt, workload, xs):
     pair_roof = {"bound": "hbm", "kernel": f"k_sweep<d={d}, fp64> (one apply of the tree)",
                  "achieved": pbytes / t64 / 1e9, "peak": phbm, "peak_source": psrc,
                  "unit": "GB/s", "frac": pbytes / t64 / 1e9 / phbm,
-                 "traffic": KERNEL_TRAFFIC.get(("pairs", workload)),
-                 "traffic_source": "not captured",
-                 "ms_per_launch": t64 * 1e3, "bytes_per_launch": pbytes,
+                 "ms_per_apply": t64 * 1e3, "bytes_per_apply": pbytes,
                  "pair_flops": flops,
-                 "fp32_kernel": {"ms_per_launch": t32 * 1e3}}
+                 "fp32_kernel": {"ms_per_apply": t32 * 1e3}}
     if gmat is None:
         return pair_roof
     # the method's operator kernel: algorithmic bytes per launch are x read
@@ -742,7 +738,7 @@ def rooflines(ab, op, mat, gmat, method, dt, workload, xs):
                          else ""),
             "achieved": nbytes / tg / 1e9, "peak": hbm, "peak_source": src,
             "unit": "GB/s", "frac": nbytes / tg / 1e9 / hbm,
-            "traffic": KERNEL_TRAFFIC.get(("global", workload)),
+            "traffic": KERNEL_TRAFFIC.get(workload),
             "traffic_source": "ncu dram__bytes_read+write, one launch",
             "bytes_per_launch": nbytes, "ms_per_launch": tg * 1e3,
             "pair_kernel": pair_roof}

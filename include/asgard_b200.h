@@ -91,7 +91,16 @@ int asgk_plan_create_pairs(asgk_plan **plan, int d, int n, int num_rows,
  * indices conn[nnz*d]; factor (t, k) of a pair is the n x n block at
  * vA + conn[k]*(d*T*n*n) + (t*d + k)*n*n (the layout make_kronmult_sparse
  * writes, src/asgard_kronmult_matrix.cpp:369-393, 455-461) -- this stores
- * d indices per pair instead of d*T. */
+ * d indices per pair instead of d*T.
+ *
+ * n = 3, d >= 2: a list of at most 32768 cells that holds every connected
+ * pair of a grid once (asgk_connect_1d's connections; in the expanded form
+ * the offsets of such) is recognised when the plan is created and, above a
+ * number of pairs x terms that depends on d, applied as passes along single
+ * dimensions over vectors of the grid.  The plan then holds these vectors
+ * from its creation on: up to 768 MB, more only where one term's passes need
+ * it (device bytes: asgk_plan_info).  With too little memory for them it is
+ * applied pair by pair, like every other list. */
 int asgk_plan_create_conn(asgk_plan **plan, int d, int n, int num_rows,
                           int num_cols, int num_terms, const int64_t *row_ptr,
                           const int *col_indx, const int *conn,
@@ -105,7 +114,8 @@ int asgk_plan_create_conn(asgk_plan **plan, int d, int n, int num_rows,
  * list written straight into the plan.  vA in the per-1D-connection layout
  * of asgk_plan_create_conn.  The same plan as asgk_build_pairs followed by
  * asgk_plan_create_conn (the same pairs in the same order), without the
- * host pass and the copy of the pair list. */
+ * host pass and the copy of the pair list, and without that function's limit
+ * on the cells of grids that are applied along single dimensions. */
 int asgk_plan_create_grid(asgk_plan **plan, int d, int n, int level,
                           int num_terms, const double *vA, int64_t vA_len);
 
