@@ -64,10 +64,12 @@ struct sweep_data
   int *last   = nullptr; // [nresults] the vectors whose sum is the product
   double *work = nullptr;
   // Whose turn with work it is: one thread enqueues at a time, and an apply
-  // on any stream waits for the one before it (done, once used is set).
+  // waits for the one before it on another stream (done, once used is set; a
+  // stream is told by its id, which unlike its handle is never used again).
   std::recursive_mutex turn;
   cudaEvent_t done = nullptr;
   bool used        = false;
+  unsigned long long by = 0; // the stream of the last apply or solve
   int nresults = 0;
   bool chains  = false; // separate chains, not a tree
   sweep_units su[6][3];
@@ -998,8 +1000,13 @@ sweep_turn::~sweep_turn()
 }
 int sweep_turn::wait(cudaStream_t s)
 {
-  if (w_ && w_->used)
+  if (w_ == nullptr)
+    return ASGK_OK;
+  unsigned long long id = 0;
+  ASGK_CUDA(cudaStreamGetId(s, &id));
+  if (w_->used && id != w_->by) // a wait of no use costs an apply 2 us
     ASGK_CUDA(cudaStreamWaitEvent(s, w_->done, 0));
+  w_->by = id;
   return ASGK_OK;
 }
 
