@@ -354,7 +354,7 @@ large_pencil(const int4 *__restrict__ recs, int rounds, const int *__restrict__ 
 // load/store pipe to 59 % (d=4 level 7) and 47 % (d=6 level 5, where DRAM moves
 // 3.4 TB/s), narrow ones wait for one chain of loads.  One FP64 apply, all
 // launches: d=4 level 7, 4 terms 254 us (5305 by the pair kernel); d=6 level
-// 5, 6 terms 2.96 ms (21.8); d=3 level 6, 2 terms, as separate chains 28 us
+// 5, 6 terms 2.96 ms (21.8); d=3 level 6, 2 terms, as separate chains 26 us
 // (129 with a kernel of a thread per output entry).  Two blocks per SM: more
 // spill the fibres (d=4 277 -> 320-500 us with three or four).
 template<int D, typename TC, typename TX>

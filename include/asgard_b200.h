@@ -167,8 +167,9 @@ int asgk_plan_kind(const asgk_plan *plan);
  * applied in one pass with the others; a term acting in m >= 2 dimensions
  * as a tree of 1D passes over the upper, whole and lower parts of its 1D
  * operators, the reference's 2^(m-1) chains of m passes with their common
- * beginnings and ends done once.  n = 3 only.  The
- * plan works with asgk_apply / asgk_apply_euler / the GMRES and Jacobi
+ * beginnings and ends done once, or on small grids as those chains side by
+ * side; such terms need num_cells * n^d < 2^31 (ASGK_ERR_UNSUPPORTED).  n = 3
+ * only.  The plan works with asgk_apply / asgk_apply_euler / the GMRES and Jacobi
  * entries like any other; asgk_plan_info's num_batch reports the neighbour
  * entries of the terms' passes (the separate chains' for those that act in
  * several dimensions) and flops 2 * n^(d+1) per entry.
