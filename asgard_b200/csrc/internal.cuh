@@ -228,10 +228,11 @@ struct jacobi_data;
 // normalisation of a recorded GMRES step's new basis vector, fused), and
 // with vcopy also vcopy = FP32(v) (the basis copy of FP32 inner solves).
 // zcopy (the line preconditioner only, else ignored): also zcopy = FP32(z),
-// the FP32 copy of x the next FP32 global apply reads
+// the FP32 copy of x the next FP32 global apply reads.  alone: not inside a
+// solve (recorded or host-driven, whose applies give the same bits)
 int jacobi_apply(jacobi_data const &jd, bool low, double *v, double *z,
                  const double *scale_state, float *vcopy, cudaStream_t s,
-                 float *zcopy = nullptr);
+                 float *zcopy = nullptr, bool alone = false);
 int jacobi_apply_handle(asgk_jacobi *pc, bool low, double *v, double *z,
                         const double *scale_state, float *vcopy,
                         cudaStream_t s, float *zcopy = nullptr);
@@ -253,7 +254,7 @@ int line_build(plan_data const &p, double dt, line_data **out, int64_t &bytes);
 void line_free(line_data *ld);
 int line_apply(line_data const &ld, bool low, double *v, double *z,
                const double *scale_state, float *vcopy, float *zcopy,
-               cudaStream_t s);
+               cudaStream_t s, bool alone);
 // the line dimensions (up to 3) into dims; returns how many
 int line_info(line_data const &ld, int *dims);
 

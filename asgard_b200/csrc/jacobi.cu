@@ -822,11 +822,11 @@ int jacobi_build(plan_data const &p, double dt, int kind, jacobi_data &jd)
 
 int jacobi_apply(jacobi_data const &jd, bool low, double *v, double *z,
                  const double *scale_state, float *vcopy, cudaStream_t s,
-                 float *zcopy)
+                 float *zcopy, bool alone)
 {
   int64_t const n = int64_t(jd.rows) * jd.ts;
   if (jd.kind == ASGK_JACOBI_LINE)
-    return line_apply(*jd.line, low, v, z, scale_state, vcopy, zcopy, s);
+    return line_apply(*jd.line, low, v, z, scale_state, vcopy, zcopy, s, alone);
   if (jd.kind == ASGK_JACOBI_KRON)
   {
     if (low)
@@ -905,7 +905,7 @@ int asgk_jacobi_apply(asgk_jacobi *pc, const double *v, double *z,
       return ASGK_ERR_INVALID;
     // without a scale state v is only read
     return asgk::jacobi_apply(pc->jd, false, const_cast<double *>(v), z, nullptr,
-                              nullptr, static_cast<cudaStream_t>(stream));
+                              nullptr, static_cast<cudaStream_t>(stream), nullptr, true);
   }
   catch (std::bad_alloc const &)
   {
@@ -927,7 +927,7 @@ int asgk_jacobi_apply_precision(asgk_jacobi *pc, int precision,
       return ASGK_ERR_INVALID;
     return asgk::jacobi_apply(pc->jd, precision == ASGK_FP32,
                               const_cast<double *>(v), z, nullptr, nullptr,
-                              static_cast<cudaStream_t>(stream));
+                              static_cast<cudaStream_t>(stream), nullptr, true);
   }
   catch (std::bad_alloc const &)
   {

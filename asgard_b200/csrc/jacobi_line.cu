@@ -387,10 +387,11 @@ constexpr int kSplitTile  = 64; // matrix rows per staged tile
 constexpr int kSplitMinM       = 64;
 constexpr int kSplitUnits      = 2 * 148 / kSplit;
 constexpr int64_t kSplitValues = 1 << 20;
-// A launch uses them while the longest pencil's chain (its matrix: cells^2)
-// is what the factor waits for, up to so many values of the vector per
-// cells^2; beyond, in recorded cycles, the clusters cost more than they save,
-// and their units run as one CTA each.  Solves without and with clusters:
+// A solve's applies use them while the longest pencil's chain (its matrix:
+// cells^2) is what the factor waits for, up to so many values of the vector
+// per cells^2; beyond, recorded cycles, which do not run the clusters beside
+// the small pencils' launch, lose by them, and their units run as one CTA
+// each.  Solves without and with clusters:
 // FP64, M line dimensions, values / longest^2 = 61 (d=4 level 4, M=2) 1.31 and
 // 1.20 ms; 30 (d=4 level 6) M=1 1.03 and 0.82; 176 (d=5 level 6) M=2 5.03 and
 // 4.15, M=1 1.55 and 1.56 (an apply 38 and 44 us); 238 (d=5 level 5) M=2 2.36
@@ -400,6 +401,13 @@ constexpr int64_t kSplitValues = 1 << 20;
 // and 2.86.
 template<typename R, int M>
 constexpr int64_t kSplitShare = (sizeof(R) == 4 ? 200 : 100) * (M > 1 ? 2 : 1);
+// An apply of its own, launched from the host, runs both side by side and uses
+// them for longer: FP32 up to kSplitValues (ratio 1427, d=6 level 4, 75 and 51
+// to 63 us); FP64 M=2 at 238 54 and 40, at 305 39 and 35, but at 1427 103 and
+// 115, and with M=1 at 176 41 and 45.
+template<typename R, int M>
+constexpr int64_t kSplitShareAlone =
+    sizeof(R) == 4 ? kSplitValues : kSplitShare<R, M> * (M > 1 ? 2 : 1);
 inline bool line_splits(int m)
 {
   return m % (4 * kSplit) == 0 && 3 * m / (4 * kSplit) <= kSplitItems;
@@ -1594,7 +1602,7 @@ template<typename R, int D, int M, int KIDX>
 int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
                   const R *inR, double *out64, R *outR, bool bj,
                   const double *sc, double *vscale, float *vc, float *zc,
-                  cudaStream_t s)
+                  cudaStream_t s, bool alone)
 {
   constexpr int NC  = ipow3l(M - 1);
   constexpr int NCP = NC == 1 ? 1 : (NC == 3 ? 4 : 12);
@@ -1620,8 +1628,8 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
     a.st_line[q] = q < M ? ipow3l(D - 1 - ld.line[q]) : 0;
   // the launches of the factor, the first on the caller's stream
   int64_t const values = int64_t(ld.rows) * ipow3l(D);
-  int const nsplit =
-      values <= kSplitShare<R, M> * f.longest * f.longest ? f.nsplit : 0;
+  int64_t const share = alone ? kSplitShareAlone<R, M> : kSplitShare<R, M>;
+  int const nsplit    = values <= share * f.longest * f.longest ? f.nsplit : 0;
   int const nlarge   = f.nunits - nsplit;
   int const max_rows = nsplit > 0 ? f.max_rows : std::max(f.max_rows, f.split_rows);
   int const max_rp   = nsplit > 0 ? f.max_rp : std::max(f.max_rp, f.split_rp);
@@ -1711,15 +1719,15 @@ int launch_factor(line_data const &ld, line_factor const &f, const double *in64,
 template<typename R, int D, int M, int KIDX>
 int factor_q(line_data const &ld, const double *in64, const R *inR, double *out64,
              R *outR, bool bj, const double *sc, double *vscale, float *vc,
-             float *zc, cudaStream_t s)
+             float *zc, cudaStream_t s, bool alone)
 {
   return launch_factor<R, D, M, KIDX>(ld, *ld.factors[KIDX], in64, inR, out64, outR,
-                                      bj, sc, vscale, vc, zc, s);
+                                      bj, sc, vscale, vc, zc, s, alone);
 }
 
 template<typename R, int D, int M>
 int apply_dm(line_data const &ld, double *v, double *z, const double *sc,
-             float *vc, float *zc, cudaStream_t s)
+             float *vc, float *zc, cudaStream_t s, bool alone)
 {
   int64_t const n = int64_t(ld.rows) * ld.ts;
   R *w0 = reinterpret_cast<R *>(ld.work);
@@ -1739,13 +1747,13 @@ int apply_dm(line_data const &ld, double *v, double *z, const double *sc,
     float *lzc        = last ? zc : nullptr;
     int rc            = ASGK_ERR_UNSUPPORTED;
     if (q == 0)
-      rc = factor_q<R, D, M, 0>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s);
+      rc = factor_q<R, D, M, 0>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s, alone);
     else if constexpr (M >= 2)
     {
       if (q == 1)
-        rc = factor_q<R, D, M, 1>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s);
+        rc = factor_q<R, D, M, 1>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s, alone);
       else if constexpr (M >= 3)
-        rc = factor_q<R, D, M, 2>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s);
+        rc = factor_q<R, D, M, 2>(ld, i64, iR, o64, oR, !first, fsc, fvs, fvc, lzc, s, alone);
     }
     if (rc)
       return rc;
@@ -1756,18 +1764,18 @@ int apply_dm(line_data const &ld, double *v, double *z, const double *sc,
 
 template<typename R, int D>
 int apply_d(line_data const &ld, double *v, double *z, const double *sc,
-            float *vc, float *zc, cudaStream_t s)
+            float *vc, float *zc, cudaStream_t s, bool alone)
 {
   switch (ld.m)
   {
-  case 1: return apply_dm<R, D, 1>(ld, v, z, sc, vc, zc, s);
+  case 1: return apply_dm<R, D, 1>(ld, v, z, sc, vc, zc, s, alone);
   case 2:
     if constexpr (D >= 2)
-      return apply_dm<R, D, 2>(ld, v, z, sc, vc, zc, s);
+      return apply_dm<R, D, 2>(ld, v, z, sc, vc, zc, s, alone);
     break;
   case 3:
     if constexpr (D >= 3)
-      return apply_dm<R, D, 3>(ld, v, z, sc, vc, zc, s);
+      return apply_dm<R, D, 3>(ld, v, z, sc, vc, zc, s, alone);
     break;
   default: break;
   }
@@ -1777,18 +1785,18 @@ int apply_d(line_data const &ld, double *v, double *z, const double *sc,
 
 int line_apply(line_data const &ld, bool low, double *v, double *z,
                const double *scale_state, float *vcopy, float *zcopy,
-               cudaStream_t s)
+               cudaStream_t s, bool alone)
 {
   auto go = [&](auto tag) -> int {
     using R = decltype(tag);
     switch (ld.d)
     {
-    case 1: return apply_d<R, 1>(ld, v, z, scale_state, vcopy, zcopy, s);
-    case 2: return apply_d<R, 2>(ld, v, z, scale_state, vcopy, zcopy, s);
-    case 3: return apply_d<R, 3>(ld, v, z, scale_state, vcopy, zcopy, s);
-    case 4: return apply_d<R, 4>(ld, v, z, scale_state, vcopy, zcopy, s);
-    case 5: return apply_d<R, 5>(ld, v, z, scale_state, vcopy, zcopy, s);
-    case 6: return apply_d<R, 6>(ld, v, z, scale_state, vcopy, zcopy, s);
+    case 1: return apply_d<R, 1>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
+    case 2: return apply_d<R, 2>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
+    case 3: return apply_d<R, 3>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
+    case 4: return apply_d<R, 4>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
+    case 5: return apply_d<R, 5>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
+    case 6: return apply_d<R, 6>(ld, v, z, scale_state, vcopy, zcopy, s, alone);
     default: return ASGK_ERR_UNSUPPORTED;
     }
   };

@@ -359,3 +359,35 @@ def test_line_jacobi_long_pencils(cuda, d, L, T):
         assert info.status == 0 and info.true_relres <= 1e-10
         xs.append(x)
     assert torch.equal(xs[0], xs[1])
+
+
+@pytest.mark.parametrize("d,L,T", [(4, 6, 4), (5, 4, 5), (5, 5, 5), (6, 4, 6)])
+def test_line_jacobi_inside_a_solve(cuda, d, L, T):
+    """One flexible GMRES step from zero gives x along M b: the apply of the
+    solves, whose launches differ from those of an apply of its own, against
+    NumPy in FP64 as above, recorded and host-driven."""
+    import asgard_b200 as ab
+    import torch
+    op = ab.SparseGridOperator.__new__(ab.SparseGridOperator)     # without the pair list
+    op.d, op.level, op.terms, op.n = d, L, T, 3
+    op.table, op.vA = ab.sparse_grid(d, L), ab.factor_values(d, L, T)
+    op.rows = op.table.shape[0]
+    op.N = op.rows * 3 ** d
+    g = op.kronmult_matrix(mode="global")
+    dt = 1e-3
+    ln = ab.JacobiPreconditioner(g, dt, kind="line")
+    b = np.random.default_rng(d + L).uniform(-1, 1, op.N)
+    expect = _line_by_eigh(op, dt, b)
+    expect /= np.linalg.norm(expect)
+    bd = torch.from_numpy(b).cuda()
+    for precision, bar in (("fp64", 1e-12), ("fp32", 1e-5)):
+        for graphs in (True, False):
+            old = ab.gmres_settings(graphs=graphs)
+            try:
+                x = torch.zeros_like(bd)
+                info = ab.simple_gmres_euler(dt, g, x, bd, 1, 1, 0.9, tol_mode="rel", precision=precision,
+                                             precond=ln)
+            finally:
+                ab.gmres_settings(**old)
+            assert info.precond_calls == 1
+            assert rel_err((x / torch.linalg.norm(x)).cpu().numpy(), expect) < bar
